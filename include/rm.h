@@ -134,7 +134,7 @@ rm_status rm_cloud_set(rm_ctx* ctx, const float* xyz, int32_t stride, const uint
 
 /* Build the spatial index (replaces KDTreeFlann::Build,
  * src/kdtree/kdtree_flann.cu:101-117 -> CudaKdTreeBuilder::buildTree,
- * kdtree_cuda_builder.h:483-599): Morton keys, radix sort, packed float4
+ * kdtree_cuda_builder.h:483-599): curve keys, radix sort, median-split leaves, float4
  * records, implicit 4-ary box tree.  Fully on the device. */
 rm_status rm_index_build(rm_ctx* ctx);
 

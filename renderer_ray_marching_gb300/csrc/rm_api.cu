@@ -202,8 +202,8 @@ void rm_ctx_destroy(rm_ctx* ctx) {
   cudaSetDevice(c.cfg.device);
   if (c.stream) cudaStreamSynchronize(c.stream);
   c.drop_graph();
-  DevBuf* bufs[] = {&c.pos, &c.rgb, &c.radii_clamped, &c.rec, &c.col, &c.perm, &c.iperm,
-                    &c.groups, &c.keys[0], &c.keys[1], &c.vals[0], &c.vals[1], &c.sort_counts,
+  DevBuf* bufs[] = {&c.pos, &c.radii_clamped, &c.rec, &c.col, &c.perm, &c.groups,
+                    &c.keys[0], &c.keys[1], &c.vals[0], &c.vals[1], &c.sort_counts,
                     &c.scan_sums, &c.scratch_bounds, &c.scalars, &c.staging_in, &c.staging_out,
                     &c.views, &c.frame_bufs, &c.queue};
   for (DevBuf* b : bufs) b->release();
@@ -240,16 +240,10 @@ rm_status rm_cloud_set(rm_ctx* ctx, const float* xyz, int32_t stride, const uint
     c.max_r = INFINITY;
     size_t np = (size_t)(n > 0 ? n : 1);
     c.pos.reserve(np * sizeof(float4));
-    c.rgb.reserve(np * sizeof(uint32_t));
     if (n > 0) {
       const float* dx = (const float*)stage_in(c, c.staging_in, xyz, (size_t)n * stride * sizeof(float), loc);
-      launch_pack_points(c, dx, stride, n);
-      const uint8_t* dr = nullptr;
-      if (rgb) {
-        // staging_in may still be read by the pack kernel: use staging_out for colours
-        dr = (const uint8_t*)stage_in(c, c.staging_out, rgb, (size_t)n * 3, loc);
-      }
-      launch_pack_colours(c, dr, n);
+      const uint8_t* dr = (const uint8_t*)stage_in(c, c.staging_out, rgb, (size_t)n * 3, loc);
+      launch_pack(c, dx, stride, dr, n);
       CK(cudaGetLastError());
       CK(cudaStreamSynchronize(c.stream));
     }

@@ -25,10 +25,12 @@ struct BackArgs {
   const int64_t* pix_base;   // per view, first pixel of the view; [n] = total
   int nviews;
   int64_t total;
+  int64_t n;                 // points in the cloud
   const float* dl_drgb;      // 3 floats per pixel
   const float* dl_ddepth;    // 1 float per pixel
   const int32_t* hit;        // cloud index per pixel, -1 = miss
-  const int32_t* iperm;      // cloud index -> sorted position
+  const float4* pos;         // cloud order
+  const float* radius;       // cloud order, clamped
   float* g_rgb;              // 3 floats per point
   float* g_xyz;              // 3 floats per point
   float* g_radius;           // 1 float per point
@@ -44,7 +46,7 @@ __device__ __forceinline__ int view_of_pixel(const int64_t* base, int n, int64_t
   return lo;
 }
 
-__global__ void __launch_bounds__(256) k_backward(IndexDev ix, BackArgs a) {
+__global__ void __launch_bounds__(256) k_backward(BackArgs a) {
   const unsigned FULL = 0xffffffffu;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -56,20 +58,19 @@ __global__ void __launch_bounds__(256) k_backward(IndexDev ix, BackArgs a) {
     float g[7] = {0, 0, 0, 0, 0, 0, 0};
     if (p < a.total) {
       h = __ldg(a.hit + p);
-      if (h >= ix.n) h = -1;  // caller-supplied index outside the cloud: ignored
+      if (h >= a.n) h = -1;  // caller-supplied index outside the cloud: ignored
       if (h >= 0) {
         int v = view_of_pixel(a.pix_base, a.nviews, p);
         const ViewDev& V = a.views[v];
         int64_t local = p - a.pix_base[v];
         int x = (int)(local % V.width), y = (int)(local / V.width);
         Ray r = make_ray(V.m, V.width, V.height, V.pane, x, y);
-        int32_t s = __ldg(a.iperm + h);
-        float4 c = __ldg(ix.rec + s);
+        const float4 c = __ldg(a.pos + h);
         double d0 = r.dx, d1 = r.dy, d2 = r.dz;
         double oc0 = (double)c.x - (double)r.ox;
         double oc1 = (double)c.y - (double)r.oy;
         double oc2 = (double)c.z - (double)r.oz;
-        double rr = c.w;
+        double rr = __ldg(a.radius + h);
         double aa = d0 * d0 + d1 * d1 + d2 * d2;
         double b = d0 * oc0 + d1 * oc1 + d2 * oc2;
         double cc = oc0 * oc0 + oc1 * oc1 + oc2 * oc2 - rr * rr;
@@ -131,10 +132,12 @@ void launch_backward(Ctx& c, const ViewDev* views_dev, int n, int64_t total_pixe
   a.pix_base = pix_base;
   a.nviews = n;
   a.total = total_pixels;
+  a.n = c.n;
   a.dl_drgb = dl_drgb;
   a.dl_ddepth = dl_ddepth;
   a.hit = hit;
-  a.iperm = c.iperm.ptr<int32_t>();
+  a.pos = c.pos.ptr<float4>();
+  a.radius = c.radii_clamped.ptr<float>();
   a.g_rgb = g_rgb;
   a.g_xyz = g_xyz;
   a.g_radius = g_radius;
@@ -142,7 +145,7 @@ void launch_backward(Ctx& c, const ViewDev* views_dev, int n, int64_t total_pixe
   int64_t cap = (int64_t)c.sm_count * 16;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  k_backward<<<(unsigned)blocks, 256, 0, c.stream>>>(c.index(), a);
+  k_backward<<<(unsigned)blocks, 256, 0, c.stream>>>(a);
 }
 
 }  // namespace rm

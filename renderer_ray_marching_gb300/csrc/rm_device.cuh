@@ -27,11 +27,12 @@ constexpr float MIN_DIST = 0.001f;  // src/common.h:7
 constexpr int MAX_LEVELS = 14;      // 4^14 leaf slots (group offsets stay 32-bit)
 constexpr int STACK = 3 * MAX_LEVELS + 4;
 constexpr int GROUP_F4 = 8;         // float4 per child group (6 used)
+constexpr float FLT_BIG = 3.402823466e+38f;  // largest finite float
 
 // Index view passed by value to kernels.
 struct IndexDev {
   const float4* rec;     // sorted records (x, y, z, radius)
-  const float4* col;     // sorted colours (r, g, b, 1)
+  const uint32_t* col;   // sorted colours (r | g << 8 | b << 16)
   const float4* groups;  // child groups: per internal node, its 4 children's boxes
   const int32_t* perm;   // sorted position -> cloud index
   int64_t n;             // points
@@ -383,7 +384,7 @@ __device__ bool knn_search(const IndexDev& ix, float qx, float qy, float qz, Lis
         }
       }
     } else {
-      float w = list_worst(L);
+      const float w = fminf(list_worst(L), FLT_BIG);  // empty boxes, at +inf, are never needed
       if (sp + 3 > STACK) return false;
       uint32_t code = (uint32_t)(lvl + 1) << 28;
       if (m3 <= w) { stk[sp] = code | (base + c3); stkd[sp] = m3; ++sp; }
@@ -408,6 +409,222 @@ __device__ bool knn_search(const IndexDev& ix, float qx, float qy, float qz, Lis
     if (!found) break;
   }
   return true;
+}
+
+// ---------------------------------------------------------------------------
+// One query per warp.
+//
+// The warp's list: lane j holds the j-th nearest point as a 64-bit key
+// (bits of d2, cloud index), so keys order exactly like (d2, cloud index),
+// and its sorted position s.  Unfilled entries have s = -1 and a key above
+// every point's.
+struct WarpList {
+  unsigned long long key;
+  int32_t s;
+  __device__ __forceinline__ float dist(int j) const {
+    return __uint_as_float(__shfl_sync(0xffffffffu, (unsigned)(key >> 32), j));
+  }
+  // empty list whose entries stand at distance `bound`
+  __device__ __forceinline__ void clear(float bound) {
+    key = ((unsigned long long)__float_as_uint(bound) << 32) | 0xffffffffu;
+    s = -1;
+  }
+  __device__ __forceinline__ void exchange(unsigned long long& k, int32_t& v, int j, bool keep_min) const {
+    const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, j);
+    const int32_t ov = __shfl_xor_sync(0xffffffffu, v, j);
+    if ((ok < k) == keep_min) {
+      k = ok;
+      v = ov;
+    }
+  }
+  // Takes one candidate per lane (d2, sorted position) where `take` is set.
+  // A few go in one by one; many are sorted by a bitonic network and merged
+  // with the list (26 exchange steps, the price of about ten insertions).
+  __device__ __forceinline__ void offer(bool take, float d2, int32_t pos, const int32_t* __restrict__ perm) {
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    unsigned todo = __ballot_sync(FULL, take);
+    if (todo == 0) return;
+    unsigned long long k = ~0ull;
+    if (take) k = ((unsigned long long)__float_as_uint(d2) << 32) | (unsigned)__ldg(perm + pos);
+    if (__popc(todo) <= 10) {
+      for (; todo; todo &= todo - 1u) {
+        const int src = __ffs(todo) - 1;
+        const unsigned long long ck = __shfl_sync(FULL, k, src);
+        const int32_t cs = __shfl_sync(FULL, pos, src);
+        const bool below = key < ck;
+        const unsigned long long uk = __shfl_up_sync(FULL, key, 1);
+        const int32_t us = __shfl_up_sync(FULL, s, 1);
+        const int at = __popc(__ballot_sync(FULL, below));
+        if (lane >= at) {
+          key = lane == at ? ck : uk;
+          s = lane == at ? cs : us;
+        }
+      }
+      return;
+    }
+#pragma unroll
+    for (int size = 2; size <= 32; size *= 2)
+#pragma unroll
+      for (int j = size / 2; j > 0; j /= 2) exchange(k, pos, j, ((lane & j) == 0) == ((lane & size) == 0));
+    // the 32 smallest of both, as a bitonic sequence
+    const unsigned long long rk = __shfl_xor_sync(FULL, k, 31);
+    const int32_t rs = __shfl_xor_sync(FULL, pos, 31);
+    if (rk < key) {
+      key = rk;
+      s = rs;
+    }
+#pragma unroll
+    for (int j = 16; j > 0; j /= 2) exchange(key, s, j, (lane & j) == 0);
+  }
+};
+
+// Pending nodes of a one-query walk, unordered: group index and box
+// distance.  Expanding a node removes it and adds at most 16.  Above
+// WPOOL_FULL entries the walk takes the newest entry, one at a time, which
+// adds at most 15 per two levels.
+constexpr int WPOOL = 384;
+constexpr int WPOOL_FULL = WPOOL - 32 - 16 * (MAX_LEVELS / 2);
+static_assert(WPOOL_FULL >= 64, "one-query pool too small");
+struct WarpPool {
+  uint32_t code[WPOOL];
+  float dist[WPOOL];
+};
+
+// The nearest points of one query (all lanes pass the same), found by the
+// whole warp.  The list arrives cleared or bounded; on return its first k
+// entries are the k nearest points within its bound.
+//
+// Best-first: every step takes the two nearest pending nodes; the walk ends
+// when none is within the k-th distance.  The 4-ary tree is read two
+// levels at a time: the four child groups of a node are consecutive, so its
+// 16 grandchildren are 512 consecutive bytes, and 32 lanes test the
+// grandchildren of two nodes at once (an odd depth takes its first step
+// alone).  Then the leaves among them are measured, 32 points at a time.
+__device__ __forceinline__ void warp_knn(const IndexDev& ix, float qx, float qy, float qz, int k, WarpList& L,
+                                         WarpPool& pool) {
+  const unsigned FULL = 0xffffffffu;
+  const float INF = __int_as_float(0x7f800000);
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  if (ix.n <= 0) return;
+  const uint32_t last_first = (uint32_t)group_offset(ix.depth - 1);  // first group of level depth-1
+  const int per = 32 / ix.leaf;                                      // leaves measured at a time
+  const int part = lane / ix.leaf, slot = lane % ix.leaf;
+  float w = L.dist(k - 1);
+  bool two = !(ix.depth & 1);
+  uint32_t G0 = 0, G1 = 0;
+  int take = 1, n = 0;
+  while (true) {
+    // children of the taken nodes
+    const bool on = two ? (lane >> 4) < take : lane < 4;
+    const uint32_t G = lane < 16 ? G0 : G1;
+    const uint32_t g = two ? 4u * G + 1u + ((lane >> 2) & 3u) : G;
+    float m = INF;
+    if (on) {
+      const float* b = reinterpret_cast<const float*>(ix.groups + (size_t)GROUP_F4 * g) + (lane & 3);
+      m = d2_box(__ldg(b), __ldg(b + 4), __ldg(b + 8), __ldg(b + 12), __ldg(b + 16), __ldg(b + 20), qx, qy, qz);
+    }
+    two = true;
+    const bool need = m <= fminf(w, FLT_BIG);  // empty boxes, at +inf, are never needed
+    const bool bottom = g >= last_first;
+    const unsigned inner = __ballot_sync(FULL, need && !bottom);
+    unsigned leaves = __ballot_sync(FULL, need && bottom);
+    if (need && !bottom) {
+      const int e = n + __popc(inner & lt);
+      pool.code[e] = 4u * g + 1u + (lane & 3u);
+      pool.dist[e] = m;
+    }
+    n += __popc(inner);
+    // leaves among them, the nearest one in the first batch
+    const uint32_t lf = (g - last_first) * 4u + (lane & 3u);
+    unsigned next = 0;
+    if (leaves) next = 1u << (__reduce_min_sync(FULL, need && bottom ? (__float_as_uint(m) & ~31u) | (unsigned)lane : ~0u) & 31u);
+    while (leaves) {
+      int src = -1;
+      for (int p = 0; p < per && leaves; ++p) {
+        if (next == 0) next = leaves & (0u - leaves);
+        if (part == p) src = __ffs(next) - 1;
+        leaves &= ~next;
+        next = 0;
+      }
+      const uint32_t f = __shfl_sync(FULL, lf, src & 31);
+      const float fm = __shfl_sync(FULL, m, src & 31);
+      const int64_t pos = (int64_t)f * ix.leaf + slot;
+      float d = FLT_BIG;
+      const bool ok = src >= 0 && fm <= w && pos < ix.n;
+      if (ok) d = d2_point(__ldg(ix.rec + pos), qx, qy, qz);
+      L.offer(ok && d <= fminf(w, FLT_BIG), d, (int32_t)pos, ix.perm);
+      w = L.dist(k - 1);
+      leaves &= __ballot_sync(FULL, m <= w);
+    }
+    __syncwarp();  // the pool's new entries
+    // next nodes: each lane's nearest of every 32nd entry, then the nearest two of those
+    if (n == 0) break;
+    if (n > WPOOL_FULL) {
+      // drop what is beyond the k-th distance
+      int kept = 0;
+      for (int i = 0; i < n; i += 32) {
+        uint32_t c = 0;
+        float d = INF;
+        if (i + lane < n) {
+          c = pool.code[i + lane];
+          d = pool.dist[i + lane];
+        }
+        const unsigned in = __ballot_sync(FULL, d <= fminf(w, FLT_BIG));
+        if ((in >> lane) & 1u) {
+          pool.code[kept + __popc(in & lt)] = c;
+          pool.dist[kept + __popc(in & lt)] = d;
+        }
+        kept += __popc(in);
+        __syncwarp();
+      }
+      n = kept;
+      if (n == 0) break;
+      if (n > WPOOL_FULL) {
+        --n;
+        G0 = pool.code[n];
+        take = 1;
+        __syncwarp();
+        continue;
+      }
+    }
+    float near = INF;
+    int at = 0;
+    for (int i = lane; i < n; i += 32) {
+      const float d = pool.dist[i];
+      if (d < near) {
+        near = d;
+        at = i;
+      }
+    }
+    const unsigned key = (__float_as_uint(near) & ~31u) | (unsigned)lane;
+    const unsigned k0 = __reduce_min_sync(FULL, key);
+    const unsigned k1 = __reduce_min_sync(FULL, key == k0 ? ~0u : key);
+    const float d0 = __shfl_sync(FULL, near, k0 & 31u), d1 = __shfl_sync(FULL, near, k1 & 31u);
+    const int a0 = __shfl_sync(FULL, at, k0 & 31u), a1 = __shfl_sync(FULL, at, k1 & 31u);
+    // one node at a time until there is a bound (so that no more than 15
+    // entries per two levels gather before); the keys are cut to 27 bits, so
+    // the second may be the nearer by less than that
+    const bool on0 = d0 <= fminf(w, FLT_BIG), on1 = k1 != ~0u && d1 <= fminf(w, FLT_BIG) && (w < INF || !on0);
+    if (!on0 && !on1) break;
+    const int hi = on0 && on1 ? max(a0, a1) : on0 ? a0 : a1, lo = on0 && on1 ? min(a0, a1) : -1;
+    take = lo >= 0 ? 2 : 1;
+    G0 = pool.code[hi];
+    G1 = lo >= 0 ? pool.code[lo] : 0;
+    __syncwarp();
+    // the last entries fill the gaps, the higher gap first
+    if (lane == 0) {
+      pool.code[hi] = pool.code[n - 1];
+      pool.dist[hi] = pool.dist[n - 1];
+      if (lo >= 0) {
+        pool.code[lo] = pool.code[n - 2];
+        pool.dist[lo] = pool.dist[n - 2];
+      }
+    }
+    n -= take;
+    __syncwarp();
+  }
 }
 
 // Per-warp shared memory of a packet traversal: pending nodes (their boxes
@@ -437,15 +654,6 @@ __device__ __forceinline__ void list_consider_unique(KSet& L, float d, int32_t s
   (void)r;
   L.consider(d, s, perm);
 }
-template <int K>
-__device__ __forceinline__ void list_consider_unique(KList<K>& L, float d, int32_t s, float r,
-                                                     const int32_t* perm) {
-  bool dup = false;
-#pragma unroll
-  for (int j = 0; j < K; ++j) dup |= (L.s[j] == s);
-  if (!dup) klist_insert<K>(L, d, s, r, perm);
-}
-
 #define RM_CSWAP_U(ka, ca, kb, cb)                 \
   do {                                             \
     if ((kb) < (ka)) {                             \
@@ -457,152 +665,20 @@ __device__ __forceinline__ void list_consider_unique(KList<K>& L, float d, int32
 // Warp packet traversal: exact k-NN of every active lane's query with one
 // walk of the tree for the whole warp.  A node is expanded when its box lies
 // within the current k-th distance of ANY active lane (one OR-reduction of
-// 4-bit votes per node), children are visited nearest-first for the leading
-// lane, pending nodes wait on a shared-memory stack and are re-tested when
-// popped (their boxes re-read from the parent's group), and a leaf's records
-// are staged once for the warp (broadcast loads) while every lane updates
-// its own list.  Lists may arrive seeded (insertions skip points already
-// present).  All 32 lanes call it with warp-uniform control flow; inactive
-// lanes only follow along.  Returns false if the stack bound or the node
-// budget was hit (neither can happen for depth <= MAX_LEVELS and an exact
-// bound).
+// 4-bit votes per node), and a leaf's records are staged once for the warp
+// (broadcast loads) while every lane updates its own list.  All 32 lanes
+// call it with warp-uniform control flow; inactive lanes only follow along.
+// Returns false if the node budget was hit (cannot happen with an exact
+// bound).  Nodes are addressed by their group's level-order index G: the
+// children of G have groups 4G + 1 + c, and a stack entry holds
+// (level << 28) | G, so no level offset is computed on the walk.
 //
-// Nodes are addressed by their group's level-order index G: the children of
-// G have groups 4G + 1 + c, and a stack entry holds (level << 28) | G, so no
-// level offset is computed on the walk.  Leaves are never pushed: they are
-// scanned in order when their parent (a node of level depth-1) is expanded.
-template <class List>
-__device__ bool packet_knn(const IndexDev& ix, bool active, float qx, float qy, float qz, List& L,
-                           PacketStack& ps, unsigned& leaves, unsigned& nodes) {
-  const unsigned FULL = 0xffffffffu;
-  const float INF = __int_as_float(0x7f800000);
-  const int lane = threadIdx.x & 31;
-  unsigned act = __ballot_sync(FULL, active);
-  if (act == 0 || ix.n <= 0) return true;
-  // the visiting order follows one lane: a central pixel of an 8x4 tile
-  // (lanes 11, 12, 19, 20) when one is active, whose nearest-first order
-  // suits its neighbours better than a corner's
-  const unsigned central = act & 0x00181800u;
-  const int leader = __ffs(central ? central : act) - 1;
-  const uint32_t last_first = (uint32_t)group_offset(ix.depth - 1);  // first group of level depth-1
-  const unsigned long long qx2 = f2_pack(qx, qx), qy2 = f2_pack(qy, qy), qz2 = f2_pack(qz, qz);
-  int sp = 0;
-  int lvl = 0;
-  uint32_t G = 0;
-  unsigned budget = PACKET_NODE_BUDGET;
-  while (true) {
-    ++nodes;
-    if (--budget == 0) return false;  // self-check: a walk this long means a broken bound
-    const float4* g = ix.groups + (size_t)GROUP_F4 * G;
-    float m0, m1, m2, m3;
-    {
-      float4 lx = __ldg(g + 0), ly = __ldg(g + 1), lz = __ldg(g + 2);
-      float4 hx = __ldg(g + 3), hy = __ldg(g + 4), hz = __ldg(g + 5);
-      d2_box4(lx, ly, lz, hx, hy, hz, qx2, qy2, qz2, m0, m1, m2, m3);
-    }
-    // needed children: one OR-reduction of every active lane's 4-bit vote
-    // (idle lanes do not vote: their bound may be +inf, and inf <= inf)
-    const float w = list_worst(L);
-    unsigned mine = 0;
-    if (active) mine = (m0 <= w ? 1u : 0u) | (m1 <= w ? 2u : 0u) | (m2 <= w ? 4u : 0u) | (m3 <= w ? 8u : 0u);
-    const unsigned needm = __reduce_or_sync(FULL, mine);
-    if (needm != 0) {
-      // visiting order (2 bits per position, nearest first for the leading
-      // lane); with one needed child any order will do
-      unsigned order = 0xE4u;  // 0, 1, 2, 3
-      if (needm & (needm - 1u)) {
-        float k0 = m0, k1 = m1, k2 = m2, k3 = m3;
-        int o0 = 0, o1 = 1, o2 = 2, o3 = 3;
-        RM_CSWAP_U(k0, o0, k1, o1);
-        RM_CSWAP_U(k2, o2, k3, o3);
-        RM_CSWAP_U(k0, o0, k2, o2);
-        RM_CSWAP_U(k1, o1, k3, o3);
-        RM_CSWAP_U(k1, o1, k2, o2);
-        order = __shfl_sync(FULL, (unsigned)o0 | ((unsigned)o1 << 2) | ((unsigned)o2 << 4) | ((unsigned)o3 << 6),
-                            leader);
-      }
-      if (lvl + 1 == ix.depth) {
-        const uint32_t lbase = (G - last_first) * 4u;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) {
-          const int c = (int)((order >> (2 * t)) & 3u);
-          if (!(needm & (1u << c))) continue;
-          // bounds may have shrunk while scanning nearer leaves
-          const float mc = c == 0 ? m0 : c == 1 ? m1 : c == 2 ? m2 : m3;
-          if (!__ballot_sync(FULL, active && mc <= list_worst(L))) continue;
-          const int64_t start = (int64_t)(lbase + c) * ix.leaf;
-          const int cnt = (int)min((int64_t)ix.leaf, ix.n - start);
-          ++leaves;
-          // one coalesced load of the leaf into shared memory, then broadcast
-          // reads (one point per iteration: the insertion is inlined at this
-          // single site, and unrolling it costs more in instruction fetch
-          // than it saves)
-          __syncwarp();
-          if (lane < cnt) ps.rec[lane] = __ldg(ix.rec + start + lane);
-          __syncwarp();
-          if (active) {
-            for (int k = 0; k < cnt; ++k) {
-              const float4 cr = ps.rec[k];
-              const float d = d2_point(cr, qx, qy, qz);
-              if (d <= list_worst(L)) list_consider_unique(L, d, (int32_t)(start + k), cr.w, ix.perm);
-            }
-          }
-        }
-      } else {
-        // descend into the nearest needed child; lanes 0-3 push the others
-        // (order position t by lane t), farthest deepest so the nearest pops first
-        unsigned om = 0;  // bit t: the child at order position t is needed
-#pragma unroll
-        for (int t = 0; t < 4; ++t) om |= ((needm >> ((order >> (2 * t)) & 3u)) & 1u) << t;
-        const int tf = __ffs(om) - 1;
-        const unsigned rest = om & (om - 1u);
-        if (sp + 3 > PSTACK) return false;
-        const uint32_t child0 = 4u * G + 1u;
-        if (lane < 4 && ((rest >> lane) & 1u)) {
-          const int slot = sp + __popc(rest >> (lane + 1));
-          ps.code[slot] = ((uint32_t)(lvl + 1) << 28) | (child0 + ((order >> (2 * lane)) & 3u));
-        }
-        sp += __popc(rest);
-        __syncwarp();
-        lvl = lvl + 1;
-        G = child0 + ((order >> (2 * tf)) & 3u);
-        continue;
-      }
-    }
-    bool found = false;
-    while (sp > 0) {
-      --sp;
-      const uint32_t code = ps.code[sp];
-      const int plvl = (int)(code >> 28);
-      const uint32_t pG = code & 0x0fffffffu;
-      // the node's box: lane (pG - 1) & 3 of its parent's group (pG - 1) >> 2
-      const float* pg = reinterpret_cast<const float*>(ix.groups + (size_t)GROUP_F4 * ((pG - 1u) >> 2));
-      const int c = (int)((pG - 1u) & 3u);
-      float md = INF;
-      if (active)
-        md = d2_box(__ldg(pg + 0 + c), __ldg(pg + 4 + c), __ldg(pg + 8 + c), __ldg(pg + 12 + c),
-                    __ldg(pg + 16 + c), __ldg(pg + 20 + c), qx, qy, qz);
-      if (__ballot_sync(FULL, active && md <= list_worst(L))) {
-        lvl = plvl;
-        G = pG;
-        found = true;
-        break;
-      }
-    }
-    __syncwarp();
-    if (!found) break;
-  }
-  return true;
-}
-
-// Best-first form of packet_knn for the marcher.  The depth-first walk
-// finishes the leading lane's subtree before anything else, so lanes whose
-// nearest points lie in another subtree keep loose bounds (and so want
-// most leaves) for much of the walk.  Here pending nodes wait in a priority
-// queue keyed by the leading lane's box distance, and the walk always
-// continues with the nearest one; the leaves of a node at level depth-1
-// are scanned when it is expanded.  A CPU simulation of both walks on
-// recorded warp steps gave about 20% fewer leaves and 12% fewer nodes.
+// The walk is best-first.  A depth-first walk finishes the leading lane's
+// subtree before anything else, so lanes whose nearest points lie in another
+// subtree keep loose bounds (and so want most leaves) for much of the walk.
+// Here pending nodes wait in a priority queue keyed by the leading lane's
+// box distance, and the walk always continues with the nearest one; the
+// leaves of a node at level depth-1 are scanned when it is expanded.
 // The queue is 32 entries in registers (lane i holds the i-th nearest);
 // the farthest entry of a full queue moves to an overflow stack in shared
 // memory, and if that fills as well the walk continues depth-first on the
@@ -688,8 +764,9 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
       d2_box4(lx, ly, lz, hx, hy, hz, qx2, qy2, qz2, m0, m1, m2, m3);
     }
     // needed children: one OR-reduction of every active lane's 4-bit vote
-    // (idle lanes do not vote: their bound may be +inf, and inf <= inf)
-    const float w = list_worst(L);
+    // (idle lanes do not vote: their bound may be +inf).  Empty boxes are at
+    // distance +inf and are never needed: their groups are not written.
+    const float w = fminf(list_worst(L), FLT_BIG);
     unsigned mine = 0;
     if (active) mine = (m0 <= w ? 1u : 0u) | (m1 <= w ? 2u : 0u) | (m2 <= w ? 4u : 0u) | (m3 <= w ? 8u : 0u);
     const unsigned needm = __reduce_or_sync(FULL, mine);

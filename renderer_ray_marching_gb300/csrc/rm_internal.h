@@ -89,11 +89,11 @@ struct Ctx {
   int depth = 0;
   int64_t nleaves = 0;
 
-  DevBuf pos;            // float4 cloud order (x, y, z, 0)
-  DevBuf rgb;            // uint32 packed rgb, cloud order
+  DevBuf pos;            // float4 cloud order (x, y, z, packed rgb)
   DevBuf radii_clamped;  // float cloud order (what rendering uses)
-  DevBuf rec, col;       // float4 sorted
-  DevBuf perm, iperm;    // int32
+  DevBuf rec;            // float4 sorted (x, y, z, clamped radius)
+  DevBuf col;            // uint32 sorted, packed rgb
+  DevBuf perm;           // int32, sorted position -> cloud index
   DevBuf groups;         // float4 child groups
   DevBuf keys[2], vals[2];
   DevBuf sort_counts, scan_sums, scratch_bounds;
@@ -122,7 +122,7 @@ struct Ctx {
   IndexDev index() const {
     IndexDev ix;
     ix.rec = rec.ptr<float4>();
-    ix.col = col.ptr<float4>();
+    ix.col = col.ptr<uint32_t>();
     ix.groups = groups.ptr<float4>();
     ix.perm = perm.ptr<int32_t>();
     ix.n = n;
@@ -138,8 +138,7 @@ struct Ctx {
 };
 
 // rm_index.cu
-void launch_pack_points(Ctx& c, const float* xyz, int stride, int64_t n);
-void launch_pack_colours(Ctx& c, const uint8_t* rgb, int64_t n);
+void launch_pack(Ctx& c, const float* xyz, int stride, const uint8_t* rgb, int64_t n);
 void launch_clamp_radii(Ctx& c, const float* in, float max_radius);
 void launch_clamp_radii_only(Ctx& c, const float* in, float max_radius);
 void launch_set_radius(Ctx& c);

@@ -12,12 +12,11 @@
 //      position; the largest of those distances bounds the new 10th distance
 //      (they are valid candidates), so its set restarts with that finite
 //      bound (KSet::restart);
-//   2. the warp walks the tree once, as a unit (packet_knn): a node is
+//   2. the warp walks the tree once, as a unit (packet_knn_bf): a node is
 //      expanded when its box lies within the current 10th distance of ANY
 //      active lane (one OR-reduction of 4-bit child votes), children are
 //      visited nearest-first for a leading lane, and pending nodes wait in a
-//      priority queue keyed by the leading lane's box distance
-//      (packet_knn_bf);
+//      priority queue keyed by the leading lane's box distance;
 //   3. a leaf's records are staged once for the whole warp (broadcast
 //      loads) and every lane updates its own sorted set, so all lanes'
 //      bounds tighten while the walk goes on.
@@ -140,8 +139,11 @@ __device__ __forceinline__ void write_result(const IndexDev& ix, const ViewArgs&
   atomicAdd(cnt + C_RAYS, 1ull);
   if (s >= 0) atomicAdd(cnt + C_HITS, 1ull);
   if (s >= 0) {
-    float4 c = __ldg(ix.col + s);
-    c.w = depth;  // colour with the depth in .w (src/ray_marching.cu:85-89)
+    // colour with the depth in .w (src/ray_marching.cu:85-89); uint8 / 255.0f
+    // as the PLY loader does (src/pointcloud.cpp:55)
+    const uint32_t u = __ldg(ix.col + s);
+    const float4 c = make_float4(__fdiv_rn((float)(u & 255u), 255.0f), __fdiv_rn((float)((u >> 8) & 255u), 255.0f),
+                                 __fdiv_rn((float)((u >> 16) & 255u), 255.0f), depth);
     if (v.rgbd) v.rgbd[pix] = c;
     if (v.hit) v.hit[pix] = __ldg(ix.perm + s);
     if (v.depth) v.depth[pix] = depth;

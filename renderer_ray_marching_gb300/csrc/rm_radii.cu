@@ -4,10 +4,10 @@
 // nearestKernel with k = 2 (kdtree_cuda_3d_index.cu:132-154, one thread per
 // query, result arrays in global memory), followed by a host loop doing 2N
 // synchronous device_reference copies for sqrt, and a separate clamp pass
-// (main.cu:144-149).  Here one kernel does the search and the sqrt for every
-// point, in index (Morton) order, so the 32 queries of a warp are spatial
-// neighbours and their tree walks touch the same groups and leaves (L1/L2
-// hits); short passes then write the results in cloud order and clamp.
+// (main.cu:144-149).  Here one kernel does the search and the sqrt for nearly
+// every point, in index order, so the queries of a warp are spatial
+// neighbours; the few that it leaves over are searched one per warp, and
+// short passes write the results in cloud order and clamp.
 #include "rm_internal.h"
 
 namespace rm {
@@ -30,56 +30,353 @@ k_radii(IndexDev ix, float max_radius, float* __restrict__ radii_out, int32_t* _
   }
 }
 
-// Packet form: a warp takes 32 consecutive sorted points (spatial
-// neighbours along the Morton curve), seeds each lane's 2-NN list with the
-// point itself and its previous and next records, and walks the tree once
-// for all 32 (packet_knn).  Same results as k_radii.
+// Region form: a warp takes 32 or 64 consecutive records (one compact piece
+// of the median-split order) as one or two chunks of 32 queries.
 //
-// Memory traffic.  Warps take their 32-point chunks from a global counter
-// in sorted order, so every resident warp works inside one window of about
-// (resident warps x 32) consecutive records -- a few MB, which stays in L2
-// while neighbouring warps re-read the same leaves.  (A grid-stride loop
-// spreads the resident warps over strides of the whole array, and their
-// leaf reads miss L2.)  Results go out in sorted order with coalesced
-// stores; k_radii_to_cloud moves them to cloud order afterwards.
+//   1. Seed: every lane measures the other 31 points of its query's chunk,
+//      which bounds all of the chunk's searches by the largest distance W.
+//   2. One walk for the region: eight pending nodes are expanded at a time,
+//      one child per lane, and each child's box is tested against the
+//      chunks' boxes grown by W.  Leaves that any chunk may need go
+//      onto a list with the mask of those chunks.
+//      A chunk that straddles a gap (two surfaces, a stray point) has a box
+//      far wider than its searches; such a chunk's children are tested again
+//      against every query's own bound before they are kept.
+//   3. Scan: per chunk, a listed leaf that lies within some lane's own bound
+//      is staged in shared memory and measured by all lanes.  A full list is
+//      scanned in mid-walk, which also tightens the W of the rest.
+//
+// The box-to-box distance is the same fma chain over per-axis gaps as
+// d2_box, and each gap is at most that of any query in the chunk, so a
+// needed leaf is never missed.
+//
+// Issue-bound (61% of the issue slots at 2M points).  One walk of the tree
+// per 32 queries, with every lane testing its own query against every box,
+// spent most of its instructions on the descent (59 expansions and 23 leaves
+// per warp in curve order).  Here an expansion tests 32 boxes at once, and
+// per chunk about 19 listed leaves are tested and 11 measured: 8.5 -> 3.7 ms
+// at 20M points, 61 -> 22 ms at 100M of uneven density, 76 -> 51 us at 100k
+// (together with the order of the records, k_blocks in rm_index.cu).
+//
+// Memory traffic.  Warps take their regions from a global counter in sorted
+// order, so all resident warps work inside one window of a few MB that
+// stays in L2.  Results go out in sorted order with coalesced stores;
+// k_radii_to_cloud moves them to cloud order afterwards.
 constexpr int RADII_WARPS = 4;
+// Chunks per region.  Two share the descent, but make half as many, longer
+// regions: 1 against 2 chunks measured 0.33 / 0.40 ms for all of
+// rm_radii_compute at 1M points, 0.97 / 0.99 at 4M, 2.26 / 2.15 at 10M and
+// 15.0 / 13.8 at 50M (4 chunks: 0.50, 1.11, 2.36, 14.6).
+constexpr int64_t RADII_SMALL = 5 << 20;
+constexpr int REGION_STACK = 512;  // depth-first, one node at a time, needs 3 entries per level beyond the last 64
+constexpr int REGION_LIST = 96;
+constexpr int REGION_SCANS = 3;  // scans of a full list, per chunk beyond the first, before a region gives up its walk
+// In squared lengths, a chunk on a surface is about 55 times as wide as its
+// largest search; well above that its box says little (REGION_WIDE).  The
+// squared distances to the nearest neighbour on an even surface are
+// exponentially distributed: one in 10^7 is over REGION_LOST medians.
+constexpr float REGION_WIDE = 1024.0f, REGION_LOST = 24.0f;
+static_assert(REGION_STACK > 64 + 3 * MAX_LEVELS, "region stack too small");
+
+template <int CHUNKS>
+struct RegionSmem {
+  uint32_t stack[REGION_STACK];
+  float box[6][REGION_LIST];     // listed leaves: box, number, chunks
+  uint32_t leaf[REGION_LIST];
+  uint32_t mask[REGION_LIST];
+  float4 rec[32];                // staged leaf
+  float4 q[32 * CHUNKS];         // queries
+  float d[32 * CHUNKS];          // nearest other point so far (Nearest); d = -1: no query
+  int32_t s[32 * CHUNKS], s2[32 * CHUNKS];
+  float cbox[6][CHUNKS];         // chunk boxes
+  float w[CHUNKS];               // largest d of the chunk
+};
+
+// Nearest other point of a query: (d, s) and s2, the point of the next
+// higher cloud index at the same distance d (-1: none).
+struct Nearest {
+  float d;
+  int32_t s, s2;
+  // a candidate with dd <= d; the query itself and points met before are skipped
+  __device__ __forceinline__ void consider(float dd, int32_t ss, int32_t self, const int32_t* __restrict__ perm) {
+    if (ss == self || ss == s || ss == s2) return;
+    if (dd < d) {
+      d = dd;
+      s = ss;
+      s2 = -1;
+    } else if (s >= 0) {  // equal distances: lower cloud indices first
+      const int32_t i = __ldg(perm + ss);
+      if (i < __ldg(perm + s)) {
+        s2 = s;
+        s = ss;
+      } else if (s2 < 0 || i < __ldg(perm + s2)) {
+        s2 = ss;
+      }
+    }
+  }
+  // cloud index of the second entry of the self-inclusive list, -1: none
+  __device__ __forceinline__ int32_t second(int64_t self, const int32_t* __restrict__ perm) const {
+    int32_t nn = s >= 0 ? __ldg(perm + s) : -1;
+    if (d == 0.0f) {  // coincident points: the second of (self, nearest, next) by cloud index
+      const int32_t i = __ldg(perm + self);
+      if (nn < i) nn = s2 >= 0 ? min(i, __ldg(perm + s2)) : i;
+    }
+    return nn;
+  }
+};
+
+// Queries left to searches of their own (k_radii_hard): sorted positions.
+struct HardList {
+  uint32_t* pos;              // room for every point
+  unsigned long long* count;
+};
+__device__ __forceinline__ void hand_over(bool mine, uint32_t s, const HardList& hard) {
+  const unsigned m = __ballot_sync(0xffffffffu, mine);
+  if (m == 0) return;
+  const int lane = threadIdx.x & 31;
+  unsigned long long at = 0;
+  if (lane == 0) at = atomicAdd(hard.count, (unsigned long long)__popc(m));
+  at = __shfl_sync(0xffffffffu, at, 0);
+  if (mine) hard.pos[at + __popc(m & ((1u << lane) - 1u))] = s;
+}
+
+// Scans the listed leaves for every chunk that may need them and refreshes
+// the chunks' W.
+template <int CHUNKS>
+__device__ void region_scan(const IndexDev& ix, RegionSmem<CHUNKS>& sm, int64_t base, int listed) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  for (int c = 0; c < CHUNKS; ++c) {
+    const float4 q = sm.q[32 * c + lane];
+    Nearest N{sm.d[32 * c + lane], sm.s[32 * c + lane], sm.s2[32 * c + lane]};
+    const int32_t self = (int32_t)(base + 32 * c + lane);
+    for (int e = 0; e < listed; ++e) {
+      if (!((sm.mask[e] >> c) & 1u)) continue;
+      const float m = d2_box(sm.box[0][e], sm.box[1][e], sm.box[2][e], sm.box[3][e], sm.box[4][e], sm.box[5][e],
+                             q.x, q.y, q.z);
+      if (!__ballot_sync(FULL, m <= N.d)) continue;
+      const int64_t start = (int64_t)sm.leaf[e] * ix.leaf;
+      const int cnt = (int)min((int64_t)ix.leaf, ix.n - start);
+      __syncwarp();
+      if (lane < cnt) sm.rec[lane] = __ldg(ix.rec + start + lane);
+      __syncwarp();
+#pragma unroll 4
+      for (int k = 0; k < cnt; ++k) {
+        const float dd = d2_point(sm.rec[k], q.x, q.y, q.z);
+        if (dd <= N.d) N.consider(dd, (int32_t)start + k, self, ix.perm);
+      }
+    }
+    sm.d[32 * c + lane] = N.d;
+    sm.s[32 * c + lane] = N.s;
+    sm.s2[32 * c + lane] = N.s2;
+    // distances are >= 0 (or -1 for no query): ordered like signed integers
+    const int w = __reduce_max_sync(FULL, __float_as_int(N.d));
+    if (lane == 0) sm.w[c] = __int_as_float(w);
+  }
+  __syncwarp();
+}
+
+__device__ __forceinline__ uint32_t ordered_bits(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return (u & 0x80000000u) ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float from_ordered(uint32_t u) {
+  return __uint_as_float((u & 0x80000000u) ? u & 0x7fffffffu : ~u);
+}
+
+template <int CHUNKS>
 __global__ void __launch_bounds__(32 * RADII_WARPS)
-k_radii_packet(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ nn_sorted,
-               unsigned long long* __restrict__ next, unsigned long long* __restrict__ err) {
-  __shared__ PacketStack stacks[RADII_WARPS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned leaves = 0, nodes = 0;
+k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ nn_sorted,
+               unsigned long long* __restrict__ next, HardList hard) {
+  constexpr int REGION = 32 * CHUNKS;
+  __shared__ RegionSmem<CHUNKS> smem[RADII_WARPS];
+  const unsigned FULL = 0xffffffffu;
+  const float INF = __int_as_float(0x7f800000);
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  RegionSmem<CHUNKS>& sm = smem[threadIdx.x >> 5];
+  const uint32_t last_first = (uint32_t)group_offset(ix.depth - 1);  // first group of level depth-1
   while (true) {
-    unsigned long long chunk = 0;
-    if (lane == 0) chunk = atomicAdd(next, 1ull);
-    const int64_t wbase = (int64_t)__shfl_sync(0xffffffffu, chunk, 0) * 32;
-    if (wbase >= ix.n) break;
-    const int64_t s = wbase + lane;
-    const bool active = s < ix.n;
-    float4 q = active ? __ldg(ix.rec + s) : make_float4(0.f, 0.f, 0.f, 0.f);
-    KList<2> L;
-    klist_init<2>(L);
-    if (active) {
-      // seeds: the point itself and both of its sorted neighbours.  The
-      // nearer neighbour bounds the search from its first node; the warp's
-      // walk is steered by its loosest lane, and a Morton jump on one side
-      // of a point rarely falls on the other (both seeds: -9% at 20M points)
-      klist_insert<2>(L, d2_point(q, q.x, q.y, q.z), (int32_t)s, q.w, ix.perm);
-      if (s + 1 < ix.n) {
-        const float4 c = __ldg(ix.rec + s + 1);
-        klist_insert<2>(L, d2_point(c, q.x, q.y, q.z), (int32_t)(s + 1), c.w, ix.perm);
+    unsigned long long region = 0;
+    if (lane == 0) region = atomicAdd(next, 1ull);
+    const int64_t base = (int64_t)__shfl_sync(FULL, region, 0) * REGION;
+    if (base >= ix.n) break;
+    // seed
+    unsigned wide = 0;  // chunks whose box is far wider than their searches
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int64_t s = base + 32 * c + lane;
+      const bool active = s < ix.n;
+      const float4 q = active ? __ldg(ix.rec + s) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      sm.q[32 * c + lane] = q;
+      __syncwarp();
+      const int cnt = (int)max((int64_t)0, min((int64_t)32, ix.n - (base + 32 * c)));
+      float d = INF;
+      int at = -1;
+      bool tie = false;
+#pragma unroll 8
+      for (int k = 0; k < cnt; ++k) {
+        float dd = d2_point(sm.q[32 * c + k], q.x, q.y, q.z);
+        if (k == lane) dd = INF;
+        tie = dd < d ? false : tie || dd == d;
+        at = dd < d ? k : at;
+        d = fminf(d, dd);
       }
-      if (s >= 1) {
-        const float4 c = __ldg(ix.rec + s - 1);
-        list_consider_unique(L, d2_point(c, q.x, q.y, q.z), (int32_t)(s - 1), c.w, ix.perm);
+      Nearest N{d, at >= 0 ? (int32_t)(base + 32 * c) + at : -1, -1};
+      if (tie && at >= 0)  // equal nearest distances in the chunk: order them by cloud index
+        for (int k = 0; k < cnt; ++k) {
+          const float dd = d2_point(sm.q[32 * c + k], q.x, q.y, q.z);
+          if (dd == d) N.consider(dd, (int32_t)(base + 32 * c) + k, (int32_t)s, ix.perm);
+        }
+      if (active && cnt < 32 && base + 32 * c >= 32)  // a short last chunk: a bound from the chunk before it
+        for (int k = 1; k <= 32; ++k) {
+          const int64_t p = base + 32 * c - k;
+          const float dd = d2_point(__ldg(ix.rec + p), q.x, q.y, q.z);
+          if (dd <= N.d) N.consider(dd, (int32_t)p, (int32_t)s, ix.perm);
+        }
+      // A query far from the rest of its chunk (alone on its side of a gap):
+      // the chunk tells little about it, and it would widen the chunk's
+      // box, so it gets a search of its own.
+      float med = active ? N.d : INF;  // the chunk's median, by a sort across the lanes
+#pragma unroll
+      for (int size = 2; size <= 32; size *= 2)
+#pragma unroll
+        for (int j = size / 2; j > 0; j /= 2) {
+          const float o = __shfl_xor_sync(FULL, med, j);
+          med = ((lane & j) == 0) == ((lane & size) == 0) ? fminf(med, o) : fmaxf(med, o);
+        }
+      med = __shfl_sync(FULL, med, max(cnt - 1, 0) / 2);
+      const bool lost = active && N.d < INF && N.d > REGION_LOST * med;
+      hand_over(lost, (uint32_t)s, hard);
+      const bool here = active && !lost;
+      const float lim[6] = {q.x, q.y, q.z, q.x, q.y, q.z};
+#pragma unroll
+      for (int f = 0; f < 6; ++f) {
+        const uint32_t o = ordered_bits(here ? lim[f] : f < 3 ? INF : -INF);
+        const float v = from_ordered(f < 3 ? __reduce_min_sync(FULL, o) : __reduce_max_sync(FULL, o));
+        if (lane == 0) sm.cbox[f][c] = v;
       }
+      __syncwarp();
+      const float ex = sm.cbox[3][c] - sm.cbox[0][c], ey = sm.cbox[4][c] - sm.cbox[1][c], ez = sm.cbox[5][c] - sm.cbox[2][c];
+      const float diag2 = ex * ex + ey * ey + ez * ez;
+      sm.d[32 * c + lane] = here ? N.d : -1.0f;
+      sm.s[32 * c + lane] = N.s;
+      sm.s2[32 * c + lane] = N.s2;
+      const int w = __reduce_max_sync(FULL, __float_as_int(here ? N.d : -1.0f));
+      if (lane == 0) sm.w[c] = __int_as_float(w);
+      if (diag2 > REGION_WIDE * __int_as_float(w)) wide |= 1u << c;
     }
-    if (!packet_knn(ix, active, q.x, q.y, q.z, L, stacks[warp], leaves, nodes) && active) atomicAdd(err, 1ull);
-    if (active) {
-      // sqrt of the second entry (main.cu:111); +inf when the cloud has one point
-      r_sorted[s] = __fsqrt_rn(L.d[1]);
-      nn_sorted[s] = L.s[1] >= 0 ? __ldg(ix.perm + L.s[1]) : -1;
+    if (lane == 0) sm.stack[0] = 0;
+    __syncwarp();
+    // walk
+    int sp = 1, listed = 0, scans = 0;
+    while (sp > 0) {
+      if (listed > REGION_LIST - 32) {
+        if (++scans > REGION_SCANS * (CHUNKS - 1)) {
+          // the chunks' bounds are loose as a whole (points strewn over a
+          // dense surface of other blocks): a search for every query instead
+          for (int c = 0; c < CHUNKS; ++c) {
+            hand_over(sm.d[32 * c + lane] >= 0.0f, (uint32_t)(base + 32 * c + lane), hard);
+            sm.d[32 * c + lane] = -1.0f;
+          }
+          listed = 0;
+          break;
+        }
+        region_scan(ix, sm, base, listed);
+        listed = 0;
+      }
+      const int take = sp < REGION_STACK - 64 - 3 * MAX_LEVELS ? min(sp, 8) : 1;
+      const int slot = lane >> 2, ch = lane & 3;
+      uint32_t G = 0, need = 0;
+      float b[6] = {};
+      if (slot < take) {
+        G = sm.stack[sp - 1 - slot];
+        const float* g = reinterpret_cast<const float*>(ix.groups + (size_t)GROUP_F4 * G) + ch;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) b[f] = __ldg(g + 4 * f);
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) {
+          const float gx = fmaxf(fmaxf(__fsub_rn(b[0], sm.cbox[3][c]), __fsub_rn(sm.cbox[0][c], b[3])), 0.0f);
+          const float gy = fmaxf(fmaxf(__fsub_rn(b[1], sm.cbox[4][c]), __fsub_rn(sm.cbox[1][c], b[4])), 0.0f);
+          const float gz = fmaxf(fmaxf(__fsub_rn(b[2], sm.cbox[5][c]), __fsub_rn(sm.cbox[2][c], b[5])), 0.0f);
+          const float m = __fmaf_rn(gz, gz, __fmaf_rn(gx, gx, __fmul_rn(gy, gy)));
+          need |= m <= fminf(sm.w[c], FLT_BIG) ? 1u << c : 0u;  // empty boxes, at +inf, never
+        }
+      }
+      for (unsigned todo = __ballot_sync(FULL, need & wide); todo; todo &= todo - 1u) {
+        const int src = __ffs(todo) - 1;
+        float o[6];
+#pragma unroll
+        for (int f = 0; f < 6; ++f) o[f] = __shfl_sync(FULL, b[f], src);
+        for (unsigned cs = __shfl_sync(FULL, need & wide, src); cs; cs &= cs - 1u) {
+          const int c = __ffs(cs) - 1;
+          const float4 q = sm.q[32 * c + lane];
+          const float m = d2_box(o[0], o[1], o[2], o[3], o[4], o[5], q.x, q.y, q.z);
+          if (!__ballot_sync(FULL, m <= sm.d[32 * c + lane]) && lane == src) need &= ~(1u << c);
+        }
+      }
+      sp -= take;
+      const bool bottom = G >= last_first;
+      const uint32_t leaf = (G - last_first) * 4u + ch;
+      if (bottom && need) {
+        // the chunk's own leaves were measured by the seed
+        const uint64_t own = (uint64_t)leaf * (uint32_t)ix.leaf - (uint64_t)base;
+        if (own < REGION) need &= ~(1u << (own / 32));
+      }
+      const unsigned inner = __ballot_sync(FULL, need && !bottom), leaves = __ballot_sync(FULL, need && bottom);
+      __syncwarp();  // every lane has read its stack entry
+      if (need) {
+        if (!bottom) {
+          sm.stack[sp + __popc(inner & lt)] = 4u * G + 1u + ch;
+        } else {
+          const int e = listed + __popc(leaves & lt);
+#pragma unroll
+          for (int f = 0; f < 6; ++f) sm.box[f][e] = b[f];
+          sm.leaf[e] = leaf;
+          sm.mask[e] = need;
+        }
+      }
+      sp += __popc(inner);
+      listed += __popc(leaves);
+      __syncwarp();
     }
+    region_scan(ix, sm, base, listed);
+    for (int c = 0; c < CHUNKS; ++c) {
+      const int64_t s = base + 32 * c + lane;
+      const float d = sm.d[32 * c + lane];
+      if (d < 0.0f) continue;  // no query, or handed over
+      const int32_t p = sm.s[32 * c + lane], p2 = sm.s2[32 * c + lane];
+      // sqrt of the second entry of the self-inclusive list (main.cu:111);
+      // +inf when the cloud has one point
+      r_sorted[s] = __fsqrt_rn(d);
+      nn_sorted[s] = Nearest{d, p, p2}.second(s, ix.perm);
+    }
+    __syncwarp();
+  }
+}
+
+// The queries that the regions handed over, one per warp.
+__global__ void __launch_bounds__(32 * RADII_WARPS)
+k_radii_hard(IndexDev ix, HardList hard, float* __restrict__ r_sorted, int32_t* __restrict__ nn_sorted) {
+  __shared__ WarpPool pools[RADII_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned long long count = *hard.count;
+  for (unsigned long long t = blockIdx.x * RADII_WARPS + warp; t < count; t += (unsigned long long)gridDim.x * RADII_WARPS) {
+    const int32_t self = (int32_t)hard.pos[t];
+    const float4 q = __ldg(ix.rec + self);
+    // its three nearest hold the two nearest others, and itself (unless three
+    // other points coincide with it)
+    WarpList L;
+    L.clear(__int_as_float(0x7f800000));
+    warp_knn(ix, q.x, q.y, q.z, 3, L, pools[warp]);
+    const int a = __shfl_sync(0xffffffffu, L.s, 0) == self ? 1 : 0;
+    const int b = __shfl_sync(0xffffffffu, L.s, a + 1) == self ? a + 2 : a + 1;
+    const float da = L.dist(a), db = L.dist(b);
+    const int32_t sa = __shfl_sync(0xffffffffu, L.s, a), sb = __shfl_sync(0xffffffffu, L.s, b);
+    if (lane == 0) {
+      r_sorted[self] = __fsqrt_rn(da);
+      nn_sorted[self] = Nearest{da, sa, db == da ? sb : -1}.second(self, ix.perm);
+    }
+    __syncwarp();
   }
 }
 
@@ -112,21 +409,30 @@ __global__ void k_radii_to_cloud(const float* __restrict__ r_sorted, const int32
   }
 }
 
-template <int K>
-__global__ void __launch_bounds__(128)
+// General k-NN (k <= 32): one query per warp, the k nearest in the warp's
+// lanes (warp_knn).  The queries come in any order, so 32 of them in one
+// warp would share nothing: one query per lane, with its list in that lane's
+// registers, took 27.3 ms for 500k unsorted queries (k = 10, 2M points, in
+// divergent walks) where this takes 1.3, and 570 us for 1000 queries (k = 1,
+// 100k points, the latency of the longest walk) where this takes 32.
+// Issue-bound for many queries, latency-bound for few (about 8 expansions and
+// 5 batches of leaves, one after the other).
+constexpr int KNN_WARPS = 4;
+__global__ void __launch_bounds__(32 * KNN_WARPS)
 k_knn(IndexDev ix, const float* __restrict__ q, int stride, int64_t m, int k,
-      int32_t* __restrict__ idx_out, float* __restrict__ d2_out, unsigned long long* __restrict__ err) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < m;
-       t += (int64_t)gridDim.x * blockDim.x) {
+      int32_t* __restrict__ idx_out, float* __restrict__ d2_out) {
+  __shared__ WarpPool pools[KNN_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t t = blockIdx.x * (int64_t)KNN_WARPS + warp; t < m; t += (int64_t)gridDim.x * KNN_WARPS) {
     const float* p = q + t * stride;
-    KList<K> L;
-    klist_init<K>(L);
-    if (!knn_search(ix, p[0], p[1], p[2], L)) atomicAdd(err, 1ull);
-    for (int j = 0; j < k; ++j) {
-      int32_t s = L.s[j];
-      idx_out[t * k + j] = s >= 0 ? __ldg(ix.perm + s) : -1;
-      d2_out[t * k + j] = L.d[j];
+    WarpList L;
+    L.clear(__int_as_float(0x7f800000));
+    warp_knn(ix, __ldg(p), __ldg(p + 1), __ldg(p + 2), k, L, pools[warp]);
+    if (lane < k) {
+      idx_out[t * k + lane] = L.s >= 0 ? (int32_t)(unsigned)L.key : -1;
+      d2_out[t * k + lane] = __uint_as_float((unsigned)(L.key >> 32));
     }
+    __syncwarp();
   }
 }
 
@@ -148,14 +454,22 @@ void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
     float* r_sorted = c.keys[0].ptr<float>();
     int32_t* nn_sorted = c.keys[1].ptr<int32_t>();
     unsigned long long* next = c.queue.ptr<unsigned long long>() + 1;
-    CK(cudaMemsetAsync(next, 0, sizeof(unsigned long long), c.stream));
-    int per_sm = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_radii_packet, 32 * RADII_WARPS, 0));
-    const int64_t chunks = (c.n + 31) / 32;
-    int64_t grid = (int64_t)c.sm_count * (per_sm > 0 ? per_sm : 1);
-    const int64_t need = (chunks + RADII_WARPS - 1) / RADII_WARPS;
-    if (grid > need) grid = need;
-    k_radii_packet<<<(unsigned)grid, 32 * RADII_WARPS, 0, c.stream>>>(c.index(), r_sorted, nn_sorted, next, err);
+    // [1] region counter, [2] handed-over queries (positions in the sort's
+    // value buffer, free like its key buffers)
+    const HardList hard{c.vals[0].ptr<uint32_t>(), next + 1};
+    CK(cudaMemsetAsync(next, 0, 2 * sizeof(unsigned long long), c.stream));
+    auto go = [&](auto kern, int chunks) {
+      int per_sm = 0;
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * RADII_WARPS, 0));
+      const int64_t regions = (c.n + 32 * chunks - 1) / (32 * chunks);
+      int64_t grid = (int64_t)c.sm_count * (per_sm > 0 ? per_sm : 1);
+      const int64_t need = (regions + RADII_WARPS - 1) / RADII_WARPS;
+      if (grid > need) grid = need;
+      kern<<<(unsigned)grid, 32 * RADII_WARPS, 0, c.stream>>>(c.index(), r_sorted, nn_sorted, next, hard);
+    };
+    if (c.n < RADII_SMALL) go(k_radii_region<1>, 1);
+    else go(k_radii_region<2>, 2);
+    k_radii_hard<<<(unsigned)(c.sm_count * 8), 32 * RADII_WARPS, 0, c.stream>>>(c.index(), hard, r_sorted, nn_sorted);
     const int g = blocks_for(c, c.n, 256);
     const int32_t* perm = c.perm.ptr<int32_t>();
     if (radii_out)
@@ -172,13 +486,10 @@ void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
 }
 
 void launch_knn(Ctx& c, const float* q, int stride, int64_t m, int k, int32_t* idx, float* d2) {
-  unsigned long long* err = c.scalars.ptr<unsigned long long>() + 8;
-  int b = blocks_for(c, m, 128);
-  IndexDev ix = c.index();
-  if (k <= 2) k_knn<2><<<b, 128, 0, c.stream>>>(ix, q, stride, m, k, idx, d2, err);
-  else if (k <= 10) k_knn<10><<<b, 128, 0, c.stream>>>(ix, q, stride, m, k, idx, d2, err);
-  else if (k <= 16) k_knn<16><<<b, 128, 0, c.stream>>>(ix, q, stride, m, k, idx, d2, err);
-  else k_knn<32><<<b, 128, 0, c.stream>>>(ix, q, stride, m, k, idx, d2, err);
+  int64_t b = (m + KNN_WARPS - 1) / KNN_WARPS;
+  const int64_t cap = (int64_t)c.sm_count * 64;
+  if (b > cap) b = cap;
+  k_knn<<<(unsigned)b, 32 * KNN_WARPS, 0, c.stream>>>(c.index(), q, stride, m, k, idx, d2);
 }
 
 }  // namespace rm

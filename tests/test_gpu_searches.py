@@ -1,0 +1,67 @@
+"""The index's searches against the oracle at the sizes where they change
+form: blocks of 1024 points and their tails, chunks of 32 queries, one and
+two chunks per warp, exact ties and coincident points, and clouds whose
+sorted neighbours say little about the nearest ones (strays over a dense
+surface, clusters far apart), for every leaf size."""
+import numpy as np
+import pytest
+
+import oracle
+from renderer_ray_marching_gb300 import Renderer, synthetic as syn
+
+pytestmark = pytest.mark.gpu
+
+
+def _cloud(kind, n):
+    rng = np.random.default_rng(n)
+    if kind == "room":
+        return syn.make_scene(n, n_boxes=3, seed=n).xyz
+    if kind == "grid":  # nearly every distance is shared
+        return (rng.integers(0, 24, (n, 3)) * 0.125).astype(np.float32)
+    if kind == "twins":  # half of the points coincide with others
+        xyz = rng.random((n, 3)).astype(np.float32)
+        xyz[rng.integers(0, n, n // 2)] = xyz[rng.integers(0, n, n // 2)]
+        return xyz
+    if kind == "strays":  # a dense slab and a thin layer of points above it
+        xyz = rng.random((n, 3)) * [4.0, 4.0, 0.004]
+        xyz[: n // 50, 2] += 0.01
+        return xyz.astype(np.float32)
+    centres = rng.uniform(-500.0, 500.0, (max(1, n // 20), 3))  # clusters
+    return (centres[rng.integers(0, len(centres), n)] + rng.normal(0.0, 0.01, (n, 3))).astype(np.float32)
+
+
+@pytest.mark.parametrize("kind", ["room", "grid", "twins", "strays", "clusters"])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 129, 1023, 1025, 4099, 70001])
+def test_radii_and_knn(kind, n):
+    xyz = _cloud(kind, n)
+    rng = np.random.default_rng(n + 1)
+    q = np.concatenate([xyz[rng.integers(0, n, 40)], rng.uniform(-2.0, 9.0, (40, 3)).astype(np.float32)])
+    ix = oracle.Index(xyz)
+    orad, onn = ix.radii(0.0)
+    for leaf in (8, 16, 32):
+        r = Renderer(leaf_size=leaf)
+        r.set_cloud(xyz)
+        r.build_index()
+        rad, nn = r.compute_radii(0.1)
+        assert np.array_equal(rad.view(np.int32), orad.view(np.int32))
+        assert np.array_equal(nn, onn)
+        for k in (1, 2, 10, 17, 32):
+            i, d = r.knn(q, k)
+            oi, od = ix.knn(q, k)
+            assert np.array_equal(i, oi)
+            assert np.array_equal(d.view(np.int32), od.view(np.int32))
+        r.close()
+
+
+@pytest.mark.parametrize("kind", ["room", "strays", "twins"])
+@pytest.mark.parametrize("n", [(5 << 20) - 1, (5 << 20) + 33])
+def test_radii_on_both_sides_of_the_region_switch(kind, n):
+    xyz = _cloud(kind, n)
+    orad, onn = oracle.Index(xyz).radii(0.0)
+    r = Renderer()
+    r.set_cloud(xyz)
+    r.build_index()
+    rad, nn = r.compute_radii(0.1)
+    assert np.array_equal(rad.view(np.int32), orad.view(np.int32))
+    assert np.array_equal(nn, onn)
+    r.close()
