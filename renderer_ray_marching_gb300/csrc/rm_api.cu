@@ -205,7 +205,7 @@ void rm_ctx_destroy(rm_ctx* ctx) {
   DevBuf* bufs[] = {&c.pos, &c.radii_clamped, &c.rec, &c.col, &c.perm, &c.groups,
                     &c.keys[0], &c.keys[1], &c.vals[0], &c.vals[1], &c.sort_counts,
                     &c.scan_sums, &c.scratch_bounds, &c.scalars, &c.staging_in, &c.staging_out,
-                    &c.views, &c.frame_bufs, &c.queue};
+                    &c.views, &c.frame_bufs, &c.queue, &c.tail};
   for (DevBuf* b : bufs) b->release();
   if (c.pinned_views) cudaFreeHost(c.pinned_views);
   if (c.ev0) cudaEventDestroy(c.ev0);
@@ -325,6 +325,7 @@ rm_status rm_radii_compute(rm_ctx* ctx, float max_radius, float* radii_out, int3
       dr = radii_out ? c.staging_out.ptr<float>() : nullptr;
       dn = nn_out ? reinterpret_cast<int32_t*>(c.staging_out.ptr<float>() + n) : nullptr;
     }
+    reserve_tail(c);
     CK(cudaMemsetAsync(err_counter(c), 0, 8, c.stream));
     launch_radii(c, max_radius, dr, dn);  // also sets the records' radii
     CK(cudaGetLastError());
@@ -349,6 +350,7 @@ rm_status rm_radii_set(rm_ctx* ctx, const float* radii, int64_t n, float max_rad
     c.drop_graph();
     c.radii_clamped.reserve((size_t)(n ? n : 1) * 4);
     if (n > 0) {
+      reserve_tail(c);
       const float* d = (const float*)stage_in(c, c.staging_in, radii, (size_t)n * 4, loc);
       if (c.have_index) {
         launch_clamp_radii(c, d, max_radius);
@@ -485,7 +487,7 @@ void enqueue_batch(Ctx& c, int n, int64_t items, const rm_launch& L) {
     CK(cudaMemsetAsync(c.queue.p, 0, 8, c.stream));
     CK(cudaMemsetAsync(counters(c), 0, kCounters * 8, c.stream));
     CK(cudaMemsetAsync(err_counter(c), 0, 8, c.stream));
-    launch_render_batch(c, c.views.ptr<ViewDev>(), n, items, L, c.queue.ptr<unsigned long long>(), counters(c));
+    launch_render_batch(c, c.views.ptr<ViewDev>(), n, items, L, c.queue.ptr<unsigned long long>(), counters(c), true);
     cudaError_t e = cudaStreamEndCapture(c.stream, &g);
     if (e != cudaSuccess) throw CudaError(std::string("graph capture: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(&c.graph_exec, g, 0);

@@ -483,7 +483,7 @@ struct WarpList {
 // distance.  Expanding a node removes it and adds at most 16.  Above
 // WPOOL_FULL entries the walk takes the newest entry, one at a time, which
 // adds at most 15 per two levels.
-constexpr int WPOOL = 384;
+constexpr int WPOOL = 256;
 constexpr int WPOOL_FULL = WPOOL - 32 - 16 * (MAX_LEVELS / 2);
 static_assert(WPOOL_FULL >= 64, "one-query pool too small");
 struct WarpPool {
@@ -627,24 +627,25 @@ __device__ __forceinline__ void warp_knn(const IndexDev& ix, float qx, float qy,
   }
 }
 
-// Per-warp shared memory of a packet traversal: pending nodes (their boxes
-// are re-read from the parent's group and re-tested when popped).
+// Per-warp shared memory of a packet traversal.  Pending nodes of the
+// depth-first fallback, one staged leaf, and the queue's overflow stack; the
+// one-query walk's pool shares their place.  Two event counts are kept by
+// lane 0 (entries moved to the overflow stack; walks that fell back to
+// depth-first order) for the launch statistics.
 constexpr int PSTACK = 3 * MAX_LEVELS + 4;
 // Node expansions one packet walk may take before it gives up and reports
 // an error (far above any exact search's need; only a broken bound hits it).
 constexpr unsigned PACKET_NODE_BUDGET = 1u << 20;
-struct PacketStack {
-  uint32_t code[PSTACK];
-  float4 rec[32];  // one staged leaf (leaf size <= 32)
-};
-
-// Shared memory of the best-first walk: the depth-first stack and staged
-// leaf of PacketStack plus the queue's overflow stack, and two event counts
-// kept by lane 0 (entries moved to the overflow stack; walks that fell back
-// to depth-first order) for the launch statistics.
 constexpr int PKT_OVERFLOW = 256;
-struct PacketQueue : PacketStack {
-  uint32_t over[PKT_OVERFLOW];
+struct PacketQueue {
+  union {
+    struct {
+      float4 rec[32];  // one staged leaf (leaf size <= 32)
+      uint32_t code[PSTACK];
+      uint32_t over[PKT_OVERFLOW];
+    };
+    WarpPool pool;
+  };
   unsigned n_spill;
   unsigned n_dfs;
 };

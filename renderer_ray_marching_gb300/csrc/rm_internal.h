@@ -102,6 +102,7 @@ struct Ctx {
   DevBuf views;          // ViewDev table
   DevBuf frame_bufs;     // device outputs for host-side frames
   DevBuf queue;          // work-queue counters
+  DevBuf tail;           // rays handed to the marcher's tail kernel
 
   rm_launch launch{8, 4, 1, 8, 1};
   rm_stats stats{};
@@ -154,7 +155,9 @@ void launch_view_pane(Ctx& c, const rm_view* views_dev, int n, float* pane_out);
 void launch_render_plain(Ctx& c, const rm_view& v, float4* rgbd, int32_t* hit, float* depth,
                          int32_t* steps, unsigned long long* counters);
 void launch_render_batch(Ctx& c, ViewDev* views_dev, int n, int64_t total_items,
-                         const rm_launch& L, unsigned long long* queue, unsigned long long* counters);
+                         const rm_launch& L, unsigned long long* queue, unsigned long long* counters,
+                         bool with_tail);
+void reserve_tail(Ctx& c);
 void launch_prepare_views(Ctx& c, ViewDev* views_dev, int n, unsigned long long* counters);
 
 // rm_backward.cu

@@ -47,7 +47,9 @@
 // scale) covers float rounding of positions and distances.
 #include "rm_internal.h"
 
+#include <cmath>
 #include <cstring>
+#include <type_traits>
 
 namespace rm {
 
@@ -91,6 +93,8 @@ constexpr int regs_for_ctas(int ctas) { return (65536 / (ctas * 32 * WARPS_PER_C
 
 struct MarchParams {
   ClipBox clip;
+  int few;          // rays left at which a late item hands them to the tail kernel
+  unsigned budget;  // expansions and leaves after which any item does
   int search;  // 1: warp packet traversal, 0: one walk per lane
 };
 
@@ -111,7 +115,8 @@ struct ViewArgs {
 //           (no longer split: always 0), [10] queue entries moved to the overflow stack,
 //           [11] packet walks that fell back to depth-first order
 enum { C_STEPS, C_RAYS, C_HITS, C_BAD, C_COOP, C_SOLO, C_LEAVES, C_NODES, C_WSTEPS, C_SPLIT, C_SPILL, C_DFS,
-       C_N };
+       C_N,
+       C_TAIL = 15 };  // rays handed to the tail kernel; [14] how many of them it has taken
 
 // Per-warp shared state.  The view of the current item, the statistics and
 // each lane's ray live here rather than in registers: they are read or bumped
@@ -155,11 +160,92 @@ __device__ __forceinline__ void write_result(const IndexDev& ix, const ViewArgs&
   if (v.steps) v.steps[pix] = steps;
 }
 
+// A ray that leaves its packet: where it is, and the 10 nearest points of its
+// last step (-1: none yet), which bound the next one's search.
+struct alignas(64) TailRay {
+  int32_t view, pix;
+  float t;
+  int32_t nsteps;
+  int32_t seed[KNN];
+  int32_t unused[2];
+};
+static_assert(sizeof(TailRay) == 64, "one record per half line");
+
+// Rays handed to the tail kernel.  `cap` records; `count` may run past it
+// (rays without a record stay with their warp).
+struct TailList {
+  TailRay* rays;
+  unsigned long long* count;
+  int64_t cap;
+};
+
+// Marches one ray to its end with the whole warp searching for it.  All
+// lanes pass the same ray; lane j < KNN holds its seed j.  Same steps as a
+// packet's: the same search, the same order of the tests.  3 to 4 ns per step
+// with all warps busy, against 0.6 to 0.7 of a packet with 18 to 23 lanes;
+// but its step takes 4 us where a packet's takes 40.
+__device__ __forceinline__ void march_one(const IndexDev& ix, const ClipBox& clip, WarpSmem& sm, int32_t pix, float t,
+                                          int32_t nsteps, int32_t seed) {
+  const unsigned FULL = 0xffffffffu;
+  const float INF = __int_as_float(0x7f800000);
+  const int lane = threadIdx.x & 31;
+  const ViewArgs& v = sm.v;
+  const Ray r = make_ray(v.m, v.width, v.height, v.pane, pix % v.width, pix / v.width);
+  const float t_stop = clip_exit(r, clip);
+  const int32_t first = nsteps;
+  int32_t hit = -1;
+  bool fin = false;
+  while (!fin && !(t > t_stop)) {  // past the exit bound: a miss
+    const float px = __fmaf_rn(r.dx, t, r.ox), py = __fmaf_rn(r.dy, t, r.oy), pz = __fmaf_rn(r.dz, t, r.oz);
+    // bound as in KSet::restart: one ulp above the seeds' largest distance
+    float d = 0.0f;
+    if (lane < KNN && seed >= 0) d = d2_point(__ldg(ix.rec + seed), px, py, pz);
+    const bool full = __ballot_sync(FULL, lane < KNN && seed >= 0) == (1u << KNN) - 1u;
+    const float w = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(d)));
+    WarpList L;
+    L.clear(full && w < INF ? __uint_as_float(__float_as_uint(w) + 1u) : INF);
+    warp_knn(ix, px, py, pz, KNN, L, sm.ps.pool);
+    // the smallest sqrtf(d2) - r; the list is in (d2, cloud index) order, so
+    // the first lane that holds it is the reference's choice
+    seed = lane < KNN ? L.s : -1;
+    float val = INF;
+    if (seed >= 0) val = __fsub_rn(__fsqrt_rn(__uint_as_float((unsigned)(L.key >> 32))), __ldg(&ix.rec[seed].w));
+    float best = val == val ? val : INF;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) best = fminf(best, __shfl_xor_sync(FULL, best, off));
+    const unsigned at = __ballot_sync(FULL, seed >= 0 && val == best);
+    const int32_t s = at ? __shfl_sync(FULL, seed, __ffs(at) - 1) : -1;
+    ++nsteps;
+    t = __fadd_rn(t, best);
+    if (best < MIN_DIST) {  // src/ray_marching.cu:219-222
+      fin = true;
+      hit = s;
+    } else {
+      fin = t > r.t_far || nsteps >= MAX_STEPS;
+    }
+  }
+  if (lane == 0) {
+    write_result(ix, v, pix, hit, hit >= 0 ? t : 0.0f, nsteps, sm.cnt);
+    sm.cnt[C_SOLO] += (unsigned long long)(nsteps - first);
+  }
+  __syncwarp();
+}
+
 // Marches every ray of one item (origin x0, y0; tile_w x tile_h*rpl pixels)
 // of view v.  All 32 lanes call it.  SEARCH: 1 packet traversal, 0 per lane.
+//
+// Rays that leave the item.  A walk costs about the same for 5 lanes as for
+// 30 (it is the union of their searches, and its steps follow one another),
+// and the rays that graze an edge go on for tens of steps: with 6 or fewer
+// lanes left are 37% of the warp steps but 5% of the ray steps at 2M points.
+// Single items (rays far from everything, or spread over several surfaces)
+// took 12 ms of a view's 7, and 32 ms where the median warp of 65 small views
+// was done after 33.  So where there is a `tail` list, an item that has used
+// up its budget of expansions and leaves, and a late item with a few rays
+// left, hands its rays over; k_march_tail spreads them over all warps.
 template <int SEARCH>
 __device__ void march_item(const IndexDev& ix, int x0, int y0, int tile_w, int tile_h, int rpl,
-                           const MarchParams& mp, WarpSmem& sm) {
+                           const MarchParams& mp, WarpSmem& sm, int view, const TailList* tail, bool late) {
   const ViewArgs& v = sm.v;
   RayLanes& R = sm.ray;
   const unsigned FULL = 0xffffffffu;
@@ -167,6 +253,7 @@ __device__ void march_item(const IndexDev& ix, int x0, int y0, int tile_w, int t
   const unsigned lt = (1u << lane) - 1u;
   const int item_rays = tile_w * tile_h * rpl;
   int next = 0;
+  unsigned work = 0;
   bool has = false;
   KSet L;
   L.clear();
@@ -194,7 +281,25 @@ __device__ void march_item(const IndexDev& ix, int x0, int y0, int tile_w, int t
       next += __popc(need);
       need = __ballot_sync(FULL, !has);
     }
-    if (__ballot_sync(FULL, has) == 0) break;
+    const unsigned alive = __ballot_sync(FULL, has);
+    if (alive == 0) break;
+    if (SEARCH == 1 && tail && next >= item_rays && ((late && __popc(alive) <= mp.few) || work > mp.budget)) {
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(tail->count, (unsigned long long)__popc(alive));
+      at = __shfl_sync(FULL, at, 0) + __popc(alive & lt);
+      if (has && (int64_t)at < tail->cap) {
+        TailRay& o = tail->rays[at];
+        o.view = view;
+        o.pix = R.pix[lane];
+        o.t = R.t[lane];
+        o.nsteps = R.nsteps[lane];
+#pragma unroll
+        for (int j = 0; j < KNN; ++j) o.seed[j] = L.s[j];
+        has = false;
+      }
+      if (__ballot_sync(FULL, has) == 0) break;
+      tail = nullptr;  // the list is full: the rest stays
+    }
 
     float t = R.t[lane];
     bool stepping = has && !(t > R.t_stop[lane]);  // past the exit bound: a miss (culled)
@@ -214,6 +319,7 @@ __device__ void march_item(const IndexDev& ix, int x0, int y0, int tile_w, int t
       unsigned lv = 0, nd = 0;
       if (!packet_knn_bf(ix, stepping, px, py, pz, L, sm.ps, lv, nd) && stepping) atomicAdd(sm.cnt + C_BAD, 1ull);
       const unsigned any_step = __ballot_sync(FULL, stepping);  // every lane votes
+      work += nd + lv;
       if (lane == 0) {
         sm.cnt[C_LEAVES] += lv;
         sm.cnt[C_NODES] += nd;
@@ -259,15 +365,16 @@ __device__ __forceinline__ void clear_counters(WarpSmem& sm) {
 }
 
 // Adds the warp's statistics to the launch's counters.  Lane-steps are the
-// rays' step counts; they are reported as packet or per-lane lane-steps by
-// search mode.
+// rays' step counts, counted at a ray's end; those of march_one and of the
+// per-lane mode are reported as steps of single rays, the others as packet
+// steps.
 template <int SEARCH>
 __device__ __forceinline__ void flush_counters(WarpSmem& sm, unsigned long long* counters) {
   __syncwarp();
   const int lane = threadIdx.x & 31;
   if (lane < C_N) {
-    unsigned long long v = lane == C_COOP ? (SEARCH == 1 ? sm.cnt[C_STEPS] : 0ull)
-                         : lane == C_SOLO ? (SEARCH == 0 ? sm.cnt[C_STEPS] : 0ull)
+    unsigned long long v = lane == C_COOP ? (SEARCH == 1 ? sm.cnt[C_STEPS] - sm.cnt[C_SOLO] : 0ull)
+                         : lane == C_SOLO ? (SEARCH == 1 ? sm.cnt[C_SOLO] : sm.cnt[C_STEPS])
                          : lane == C_SPILL ? (unsigned long long)sm.ps.n_spill
                          : lane == C_DFS ? (unsigned long long)sm.ps.n_dfs
                          : sm.cnt[lane];
@@ -286,10 +393,40 @@ struct PlainArgs {
   int32_t* steps;
 };
 
+__device__ __forceinline__ void load_view(ViewArgs& v, const PlainArgs& a) {
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v.m[k] = a.m[k];
+    v.width = a.width;
+    v.height = a.height;
+    v.pane = view_pane(a.width, a.fov);
+    v.rgbd = a.rgbd;
+    v.hit = a.hit;
+    v.depth = a.depth;
+    v.steps = a.steps;
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void load_view(ViewArgs& v, const ViewDev& V) {
+  const int lane = threadIdx.x & 31;
+  __syncwarp();  // the previous item's readers of v are done
+  if (lane < 16) v.m[lane] = V.m[lane];
+  if (lane == 0) {
+    v.width = V.width;
+    v.height = V.height;
+    v.pane = V.pane;
+    v.rgbd = V.rgbd;
+    v.hit = V.hit;
+    v.depth = V.depth;
+    v.steps = V.steps;
+  }
+  __syncwarp();
+}
+
 // One warp per 8x4 tile.
 template <int SEARCH>
 __device__ __forceinline__ void plain_body(const IndexDev& ix, const PlainArgs& a, const MarchParams& mp,
-                                           unsigned long long* __restrict__ counters) {
+                                           unsigned long long* __restrict__ counters, const TailList& tail) {
   __shared__ WarpSmem smem[WARPS_PER_CTA];
   const int warp = threadIdx.x >> 5;
   int tiles_x = (a.width + 7) / 8;
@@ -298,19 +435,8 @@ __device__ __forceinline__ void plain_body(const IndexDev& ix, const PlainArgs& 
   WarpSmem& sm = smem[warp];
   clear_counters(sm);
   if (tile < tiles) {
-    if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-      for (int k = 0; k < 16; ++k) sm.v.m[k] = a.m[k];
-      sm.v.width = a.width;
-      sm.v.height = a.height;
-      sm.v.pane = view_pane(a.width, a.fov);
-      sm.v.rgbd = a.rgbd;
-      sm.v.hit = a.hit;
-      sm.v.depth = a.depth;
-      sm.v.steps = a.steps;
-    }
-    __syncwarp();
-    march_item<SEARCH>(ix, (tile % tiles_x) * 8, (tile / tiles_x) * 4, 8, 4, 1, mp, sm);
+    load_view(sm.v, a);
+    march_item<SEARCH>(ix, (tile % tiles_x) * 8, (tile / tiles_x) * 4, 8, 4, 1, mp, sm, 0, tail.cap > 0 ? &tail : nullptr, true);
   }
   flush_counters<SEARCH>(sm, counters);
 }
@@ -321,12 +447,12 @@ __device__ __forceinline__ void plain_body(const IndexDev& ix, const PlainArgs& 
 // 17.2 Mrays/s with __maxnreg__ at the same 90 registers).
 template <int MINB>
 __global__ void __launch_bounds__(32 * WARPS_PER_CTA) __maxnreg__(regs_for_ctas(MINB))
-k_march_plain(IndexDev ix, PlainArgs a, MarchParams mp, unsigned long long* __restrict__ counters) {
-  plain_body<1>(ix, a, mp, counters);
+k_march_plain(IndexDev ix, PlainArgs a, MarchParams mp, unsigned long long* __restrict__ counters, TailList tail) {
+  plain_body<1>(ix, a, mp, counters, tail);
 }
 __global__ void __launch_bounds__(32 * WARPS_PER_CTA, 4)
-k_march_plain_lane(IndexDev ix, PlainArgs a, MarchParams mp, unsigned long long* __restrict__ counters) {
-  plain_body<0>(ix, a, mp, counters);
+k_march_plain_lane(IndexDev ix, PlainArgs a, MarchParams mp, unsigned long long* __restrict__ counters, TailList tail) {
+  plain_body<0>(ix, a, mp, counters, tail);
 }
 
 // ---------------------------------------------------------------- batched
@@ -344,6 +470,7 @@ struct BatchArgs {
   const ViewDev* views;
   int nviews;
   int64_t total_items;
+  int64_t late_items;       // items at the queue's end that count as late
   int tile_w, tile_h, rpl;  // item = tile_w x (tile_h * rpl) pixels
 };
 
@@ -360,7 +487,7 @@ __device__ __forceinline__ int find_view(const ViewDev* views, int n, int64_t it
 template <int SEARCH>
 __device__ __forceinline__ void batch_body(const IndexDev& ix, const BatchArgs& a, const MarchParams& mp,
                                            unsigned long long* __restrict__ queue,
-                                           unsigned long long* __restrict__ counters) {
+                                           unsigned long long* __restrict__ counters, const TailList& tail) {
   __shared__ WarpSmem smem[WARPS_PER_CTA];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpSmem& sm = smem[warp];
@@ -373,21 +500,11 @@ __device__ __forceinline__ void batch_body(const IndexDev& ix, const BatchArgs& 
     int iv = find_view(a.views, a.nviews, (int64_t)it);
     const ViewDev& V = a.views[iv];
     int64_t local = (int64_t)it - V.tile_base;
-    __syncwarp();  // the previous item's readers of sm.v are done
-    if (lane < 16) sm.v.m[lane] = V.m[lane];
-    if (lane == 0) {
-      sm.v.width = V.width;
-      sm.v.height = V.height;
-      sm.v.pane = V.pane;
-      sm.v.rgbd = V.rgbd;
-      sm.v.hit = V.hit;
-      sm.v.depth = V.depth;
-      sm.v.steps = V.steps;
-    }
-    __syncwarp();
+    load_view(sm.v, V);
     int x0 = (int)(local % V.tiles_x) * a.tile_w;
     int y0 = (int)(local / V.tiles_x) * (a.tile_h * a.rpl);
-    march_item<SEARCH>(ix, x0, y0, a.tile_w, a.tile_h, a.rpl, mp, sm);
+    const bool late = (int64_t)it + a.late_items >= a.total_items;
+    march_item<SEARCH>(ix, x0, y0, a.tile_w, a.tile_h, a.rpl, mp, sm, iv, tail.cap > 0 ? &tail : nullptr, late);
   }
   flush_counters<SEARCH>(sm, counters);
 }
@@ -395,13 +512,36 @@ __device__ __forceinline__ void batch_body(const IndexDev& ix, const BatchArgs& 
 template <int MINB>
 __global__ void __launch_bounds__(32 * WARPS_PER_CTA) __maxnreg__(regs_for_ctas(MINB))
 k_march_batch(IndexDev ix, BatchArgs a, MarchParams mp, unsigned long long* __restrict__ queue,
-              unsigned long long* __restrict__ counters) {
-  batch_body<1>(ix, a, mp, queue, counters);
+              unsigned long long* __restrict__ counters, TailList tail) {
+  batch_body<1>(ix, a, mp, queue, counters, tail);
 }
 __global__ void __launch_bounds__(32 * WARPS_PER_CTA, 4)
 k_march_batch_lane(IndexDev ix, BatchArgs a, MarchParams mp, unsigned long long* __restrict__ queue,
-                   unsigned long long* __restrict__ counters) {
-  batch_body<0>(ix, a, mp, queue, counters);
+                   unsigned long long* __restrict__ counters, TailList tail) {
+  batch_body<0>(ix, a, mp, queue, counters, tail);
+}
+
+// The rays that left their items, one per warp, taken in the list's order.
+// VIEWS: the view table, or the plain form's one view.
+template <class VIEWS>
+__global__ void __launch_bounds__(32 * WARPS_PER_CTA, 8)
+k_march_tail(IndexDev ix, VIEWS views, ClipBox clip, unsigned long long* __restrict__ counters, TailList tail) {
+  __shared__ WarpSmem smem[WARPS_PER_CTA];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  WarpSmem& sm = smem[warp];
+  const unsigned long long count = min(*tail.count, (unsigned long long)tail.cap);
+  clear_counters(sm);
+  if constexpr (std::is_same<VIEWS, PlainArgs>::value) load_view(sm.v, views);
+  while (true) {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(tail.count - 1, 1ull);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= count) break;
+    const TailRay& o = tail.rays[t];
+    if constexpr (!std::is_same<VIEWS, PlainArgs>::value) load_view(sm.v, views[o.view]);
+    march_one(ix, clip, sm, o.pix, o.t, o.nsteps, lane < KNN ? o.seed[lane] : -1);
+  }
+  flush_counters<1>(sm, counters);
 }
 
 // ---------------------------------------------------------------- host side
@@ -425,10 +565,39 @@ static ClipBox clip_box(const Ctx& c, float max_r) {
   return e;
 }
 
-static MarchParams march_params(const Ctx& c) {
+static TailList tail_list(const Ctx& c, unsigned long long* counters) {
+  return TailList{c.tail.ptr<TailRay>(), counters + C_TAIL, (int64_t)(c.tail.cap / sizeof(TailRay))};
+}
+
+// Which rays leave their packets.  `few`: a late item's last rays (of 2, 4, 6,
+// 8, 12 the fastest for one 1067x690 view at 2M points; 6.9 -> 6.6 ms by
+// itself).  The budget counts node expansions and leaves of an item (about
+// 1000 at 2M points, 1400 at 20M); a ray costs the tail kernel about four
+// times its share of a full packet, so the budget is the larger the more
+// items a warp has to work off anyway, and with them the time in which a
+// slow one is hidden.  Measured optima: 200 at 0.12 items per resident warp
+// (160x120 pixels), 600 at 0.5, 900 at 2, 1000 at 5 (1067x690), 1400 at 17
+// (65 small views), 4000 to 6000 at 160 (24 views at 20M points).  Times
+// without -> with the tail kernel: 160x120 at 100k points 1.73 -> 0.65 ms,
+// 320x240 at 2M 3.2 -> 1.4, 1067x690 at 2M 6.9 -> 5.6, 65 small views at 1M
+// 47.7 -> 33.9, 24 views at 20M 334 -> 316.
+constexpr int FEW = 6;
+static unsigned tail_budget(const Ctx& c, int64_t items) {
+  const double per_warp = (double)items / ((double)c.sm_count * 8 * WARPS_PER_CTA);
+  return (unsigned)fmax(200.0, 650.0 * pow(per_warp, 0.38));
+}
+
+// 524,288 rays: 6 of every tile of a 1920x1080 view, and more.  When they are
+// used up, rays stay with their items.  Reserved with the radii, since a
+// render call may be under stream capture.
+void reserve_tail(Ctx& c) { c.tail.reserve((size_t)1 << 25); }
+
+static MarchParams march_params(const Ctx& c, int64_t items) {
   MarchParams mp;
   mp.clip = clip_box(c, c.max_r);
   mp.search = c.launch.search;
+  mp.few = FEW;
+  mp.budget = tail_budget(c, items);
   return mp;
 }
 
@@ -449,8 +618,9 @@ void launch_render_plain(Ctx& c, const rm_view& v, float4* rgbd, int32_t* hit, f
   a.steps = steps;
   int64_t tiles = (int64_t)((v.width + 7) / 8) * ((v.height + 3) / 4);
   unsigned grid = (unsigned)((tiles + WARPS_PER_CTA - 1) / WARPS_PER_CTA);
-  MarchParams mp = march_params(c);
-  auto go = [&](auto kern) { kern<<<grid, 32 * WARPS_PER_CTA, 0, c.stream>>>(c.index(), a, mp, counters); };
+  MarchParams mp = march_params(c, tiles);
+  const TailList tail = tail_list(c, counters);
+  auto go = [&](auto kern) { kern<<<grid, 32 * WARPS_PER_CTA, 0, c.stream>>>(c.index(), a, mp, counters, tail); };
   const int cps = c.launch.ctas_per_sm;
   if (mp.search == 1) {
     if (cps >= 8) go(k_march_plain<8>);
@@ -458,6 +628,8 @@ void launch_render_plain(Ctx& c, const rm_view& v, float4* rgbd, int32_t* hit, f
     else if (cps >= 6) go(k_march_plain<6>);
     else if (cps >= 5) go(k_march_plain<5>);
     else go(k_march_plain<4>);
+    if (tail.cap > 0)
+      k_march_tail<<<(unsigned)(c.sm_count * 8), 32 * WARPS_PER_CTA, 0, c.stream>>>(c.index(), a, mp.clip, counters, tail);
   } else {
     go(k_march_plain_lane);
   }
@@ -470,9 +642,10 @@ void launch_prepare_views(Ctx& c, ViewDev* views_dev, int n, unsigned long long*
 
 // `queue` is the work-queue counter the launch's warps pull items from (zero
 // before the launch): the context's own for rm_render_batch, the static
-// scratch's for the allocation-free entry point.
+// scratch's for the allocation-free entry point, which has no list of tail
+// rays either (with_tail false: every warp ends its own rays).
 void launch_render_batch(Ctx& c, ViewDev* views_dev, int n, int64_t total_items, const rm_launch& L,
-                         unsigned long long* queue, unsigned long long* counters) {
+                         unsigned long long* queue, unsigned long long* counters, bool with_tail) {
   BatchArgs a;
   a.views = views_dev;
   a.nviews = n;
@@ -481,9 +654,12 @@ void launch_render_batch(Ctx& c, ViewDev* views_dev, int n, int64_t total_items,
   a.tile_h = L.tile_h;
   a.rpl = L.rays_per_lane;
   int grid = c.sm_count * (L.ctas_per_sm > 0 ? L.ctas_per_sm : 4);
-  MarchParams mp = march_params(c);
+  a.late_items = (int64_t)grid * WARPS_PER_CTA * 2;
+  MarchParams mp = march_params(c, total_items);
+  TailList tail = tail_list(c, counters);
+  if (!with_tail) tail.cap = 0;
   auto go = [&](auto kern) {
-    kern<<<grid, 32 * WARPS_PER_CTA, 0, c.stream>>>(c.index(), a, mp, queue, counters);
+    kern<<<grid, 32 * WARPS_PER_CTA, 0, c.stream>>>(c.index(), a, mp, queue, counters, tail);
   };
   const int cps = L.ctas_per_sm;
   if (mp.search == 1) {
@@ -492,6 +668,9 @@ void launch_render_batch(Ctx& c, ViewDev* views_dev, int n, int64_t total_items,
     else if (cps >= 6) go(k_march_batch<6>);
     else if (cps >= 5) go(k_march_batch<5>);
     else go(k_march_batch<4>);
+    if (tail.cap > 0)
+      k_march_tail<<<(unsigned)(c.sm_count * 8), 32 * WARPS_PER_CTA, 0, c.stream>>>(c.index(), (const ViewDev*)views_dev,
+                                                                                    mp.clip, counters, tail);
   } else {
     go(k_march_batch_lane);
   }

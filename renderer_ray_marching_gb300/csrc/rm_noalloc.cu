@@ -118,7 +118,7 @@ extern "C" rm_status rm_render_batch_noalloc(rm_ctx* ctx, const rm_view* views, 
   if (e == cudaSuccess) e = cudaMemsetAsync(base, 0, kHeaderBytes, c.stream);
   if (e != cudaSuccess) return fail(c, RM_ERR_CUDA, cudaGetErrorString(e));
   launch_prepare_views(c, views_dev, n, counters);
-  launch_render_batch(c, views_dev, n, items, L, queue, counters);
+  launch_render_batch(c, views_dev, n, items, L, queue, counters, false);
   e = cudaGetLastError();
   unsigned long long bad = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, counters + 3, sizeof(bad), cudaMemcpyDeviceToHost, c.stream);

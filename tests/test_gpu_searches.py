@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import oracle
-from renderer_ray_marching_gb300 import Renderer, synthetic as syn
+from renderer_ray_marching_gb300 import Renderer, synthetic as syn, views_from_specs
 
 pytestmark = pytest.mark.gpu
 
@@ -64,4 +64,30 @@ def test_radii_on_both_sides_of_the_region_switch(kind, n):
     rad, nn = r.compute_radii(0.1)
     assert np.array_equal(rad.view(np.int32), orad.view(np.int32))
     assert np.array_equal(nn, onn)
+    r.close()
+
+
+@pytest.mark.parametrize("n,size", [(7, (40, 24)), (3000, (8, 4)), (3000, (161, 119)), (60_000, (900, 610)),
+                                    (20_000, (3600, 2400))])
+def test_rays_that_leave_their_packets(n, size):
+    """Packets hand rays to the tail kernel after a budget that grows with the
+    launch (the largest view also overruns the list of such rays); the march
+    of every ray alone (search 0) gives the same images."""
+    sc = syn.make_scene(n, n_boxes=6, seed=n)
+    views = views_from_specs(syn.make_views(2, seed=4, boxes=sc.boxes, resolutions=[size]))
+    r = Renderer()
+    r.set_cloud(sc.xyz, sc.rgb)
+    r.build_index()
+    r.compute_radii(0.3)
+    fields = ("rgbd", "hit", "depth", "steps")
+    plain = [r.render(v, outputs=fields) for v in views]
+    if n >= 3000 and size != (8, 4):
+        assert r.stats()["solo_steps"] > 0 and r.stats()["packet_steps"] > 0
+    batch = r.render_batch(views, outputs=fields, device=False)
+    r.set_launch(search=0, ctas_per_sm=4)
+    for v, p, b in zip(views, plain, batch):
+        alone = r.render(v, outputs=fields)
+        for f in fields:
+            assert np.array_equal(alone[f].view(np.int32), p[f].view(np.int32)), f
+            assert np.array_equal(alone[f].view(np.int32), b[f].view(np.int32)), f
     r.close()
