@@ -8,14 +8,27 @@
 // nearest spheres, so it differs from this analytic surrogate by less than
 // MIN_DIST plus one step; the surrogate is what is differentiated.
 //
-// Per pixel the kernel recomputes the ray exactly as the forward did,
-// evaluates t and its gradient in double precision (t = (b - sqrt(disc))/a
-// with a = |d|^2, b = d.(c - o), disc = b^2 - a(|c - o|^2 - r^2); the FP64
-// evaluation keeps the millimetre-scale discriminant of metre-scale
-// operands accurate), scales by the incoming dL/ddepth and accumulates into
-// float32 per-point gradients.  Pixels of a warp that share a hit point are
-// reduced in registers first (__match_any_sync), so each point receives one
-// atomic per warp and channel.
+// Per pixel the kernel recomputes the ray exactly as the forward did and
+// evaluates the gradient of t = (b - sqrt(disc)) / a, with a = |d|^2,
+// b = d.(c - o) and disc = a r^2 - |q|^2 for q = d x (c - o) (Lagrange's
+// identity for b^2 - a (|c - o|^2 - r^2)):
+//   dt/dc = (d - (d x q) / sqrt(disc)) / a,   dt/dr = -r / sqrt(disc).
+// It scales by the incoming dL/ddepth and accumulates into float32 per-point
+// gradients.  A warp's pixels are neighbours in a row; runs of them that share
+// a hit point are summed in registers first, so each run costs one atomic per
+// channel.
+//
+// Arithmetic.  A millimetre-scale discriminant of metre-scale operands needs
+// more than float32.  sm_103a has one FP64 unit for 64 FP32 lanes, and in
+// FP64 this kernel was bound by it: 1.44 ms for 16 views of 1067x690, now
+// 0.27 (issue-bound, 72% of the slots, 650 instructions per 32 pixels).  Here
+// every value is an unevaluated sum of two floats (about 48 bits, T. J.
+// Dekker's double-length arithmetic with fma products), and the cancellation
+// is taken out of the formula instead: q is as small as the ray's distance
+// from the centre, so disc = a r^2 - |q|^2 is good to 1e-10 of r^2, where
+// b^2 - a (...) in FP64 carries an error of 1e-15 b^2, 1e-9 of a
+// millimetre's square at 3 m.  Coordinates or radii outside the range where
+// floats hold such products keep FP64.
 #include "rm_internal.h"
 
 namespace rm {
@@ -46,6 +59,100 @@ __device__ __forceinline__ int view_of_pixel(const int64_t* base, int n, int64_t
   return lo;
 }
 
+// ---------------------------------------------------------------- two floats
+// hi + lo with |lo| <= ulp(hi) / 2 after a sum.
+struct Two {
+  float hi, lo;
+};
+__device__ __forceinline__ Two quick_two(float a, float b) {  // |a| >= |b|
+  const float s = __fadd_rn(a, b);
+  return Two{s, __fsub_rn(b, __fsub_rn(s, a))};
+}
+__device__ __forceinline__ Two two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+  return Two{s, __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t))};
+}
+__device__ __forceinline__ Two two_prod(float a, float b) {
+  const float p = __fmul_rn(a, b);
+  return Two{p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ Two neg(Two a) { return Two{-a.hi, -a.lo}; }
+// error 2^-47 (|a| + |b|)
+__device__ __forceinline__ Two add(Two a, Two b) {
+  const Two s = two_sum(a.hi, b.hi);
+  return quick_two(s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)));
+}
+// products, not normalised: |lo| <= 2 ulp(hi)
+__device__ __forceinline__ Two mul(Two a, float b) {
+  const Two p = two_prod(a.hi, b);
+  return Two{p.hi, __fmaf_rn(a.lo, b, p.lo)};
+}
+__device__ __forceinline__ Two mul(Two a, Two b) {
+  const Two p = two_prod(a.hi, b.hi);
+  return Two{p.hi, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.lo, p.lo))};
+}
+__device__ __forceinline__ float rounded(Two a) { return __fadd_rn(a.hi, a.lo); }
+// 1 / sqrt(a) and 1 / a: a float start and one Newton step
+__device__ __forceinline__ Two inv_sqrt(Two a) {
+  const float y = rsqrtf(a.hi);
+  const Two e = add(Two{1.0f, 0.0f}, neg(mul(a, two_prod(y, y))));
+  return quick_two(y, __fmul_rn(__fmul_rn(0.5f, y), e.hi));
+}
+__device__ __forceinline__ Two inv(Two a) {
+  const float y = __frcp_rn(a.hi);
+  const Two e = add(Two{1.0f, 0.0f}, neg(mul(a, y)));
+  return quick_two(y, __fmul_rn(y, e.hi));
+}
+
+// Gradient of the entry distance, times `ld`: out[0..2] by the centre, [3] by
+// the radius.  oc: from the ray's origin to the centre.
+__device__ __forceinline__ void entry_gradient(const Ray& r, const float4& c, float rad, float ld, float* out) {
+  const float d[3] = {r.dx, r.dy, r.dz};
+  const Two oc[3] = {two_sum(c.x, -r.ox), two_sum(c.y, -r.oy), two_sum(c.z, -r.oz)};
+  const float far = fmaxf(fmaxf(fabsf(oc[0].hi), fabsf(oc[1].hi)), fabsf(oc[2].hi));
+  if (far < 1048576.0f && rad < 1048576.0f && (rad >= 1e-9f || rad == 0.0f)) {
+    Two q[3], n[3];
+    Two aa = two_prod(d[0], d[0]);
+    aa = add(aa, two_prod(d[1], d[1]));
+    aa = add(aa, two_prod(d[2], d[2]));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int j = (i + 1) % 3, k = (i + 2) % 3;
+      q[i] = add(mul(oc[k], d[j]), neg(mul(oc[j], d[k])));
+    }
+    Two disc = mul(aa, two_prod(rad, rad));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) disc = add(disc, neg(mul(q[i], q[i])));
+    const Two ia = mul(inv(aa), ld);
+    if (disc.hi > 0.0f) {
+      const Two is = inv_sqrt(disc);
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const int j = (i + 1) % 3, k = (i + 2) % 3;
+        n[i] = add(mul(q[k], d[j]), neg(mul(q[j], d[k])));
+        out[i] = rounded(mul(add(Two{d[i], 0.0f}, neg(mul(n[i], is))), ia));
+      }
+      out[3] = -rounded(mul(is, two_prod(rad, ld)));
+    } else {
+#pragma unroll
+      for (int i = 0; i < 3; ++i) out[i] = rounded(mul(ia, d[i]));
+      out[3] = 0.0f;
+    }
+    return;
+  }
+  const double d0 = r.dx, d1 = r.dy, d2 = r.dz, rr = rad;
+  const double oc0 = (double)c.x - (double)r.ox, oc1 = (double)c.y - (double)r.oy, oc2 = (double)c.z - (double)r.oz;
+  const double a2 = d0 * d0 + d1 * d1 + d2 * d2, b = d0 * oc0 + d1 * oc1 + d2 * oc2;
+  const double disc = b * b - a2 * (oc0 * oc0 + oc1 * oc1 + oc2 * oc2 - rr * rr);
+  const double s = (double)ld / a2;
+  const double is = disc > 0.0 ? 1.0 / sqrt(disc) : 0.0;
+  const bool in = disc > 0.0;
+  out[0] = (float)((in ? d0 - (b * d0 - a2 * oc0) * is : d0) * s);
+  out[1] = (float)((in ? d1 - (b * d1 - a2 * oc1) * is : d1) * s);
+  out[2] = (float)((in ? d2 - (b * d2 - a2 * oc2) * is : d2) * s);
+  out[3] = in ? (float)((double)ld * (-rr * is)) : 0.0f;
+}
+
 __global__ void __launch_bounds__(256) k_backward(BackArgs a) {
   const unsigned FULL = 0xffffffffu;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -55,71 +162,45 @@ __global__ void __launch_bounds__(256) k_backward(BackArgs a) {
   for (int64_t wbase = warp_first; wbase < a.total; wbase += stride) {
     int64_t p = wbase + (threadIdx.x & 31);
     int32_t h = -1;
+    const int v0 = view_of_pixel(a.pix_base, a.nviews, wbase);  // the warp's first pixel's, same for all lanes
     float g[7] = {0, 0, 0, 0, 0, 0, 0};
     if (p < a.total) {
       h = __ldg(a.hit + p);
       if (h >= a.n) h = -1;  // caller-supplied index outside the cloud: ignored
       if (h >= 0) {
-        int v = view_of_pixel(a.pix_base, a.nviews, p);
+        int v = v0;
+        while (p >= a.pix_base[v + 1]) ++v;
         const ViewDev& V = a.views[v];
-        int64_t local = p - a.pix_base[v];
-        int x = (int)(local % V.width), y = (int)(local / V.width);
-        Ray r = make_ray(V.m, V.width, V.height, V.pane, x, y);
-        const float4 c = __ldg(a.pos + h);
-        double d0 = r.dx, d1 = r.dy, d2 = r.dz;
-        double oc0 = (double)c.x - (double)r.ox;
-        double oc1 = (double)c.y - (double)r.oy;
-        double oc2 = (double)c.z - (double)r.oz;
-        double rr = __ldg(a.radius + h);
-        double aa = d0 * d0 + d1 * d1 + d2 * d2;
-        double b = d0 * oc0 + d1 * oc1 + d2 * oc2;
-        double cc = oc0 * oc0 + oc1 * oc1 + oc2 * oc2 - rr * rr;
-        double disc = b * b - aa * cc;
-        double gc0, gc1, gc2, gr;
-        double ia = 1.0 / aa;
-        if (disc > 0.0) {
-          double is = 1.0 / sqrt(disc);
-          gc0 = (d0 - (b * d0 - aa * oc0) * is) * ia;
-          gc1 = (d1 - (b * d1 - aa * oc1) * is) * ia;
-          gc2 = (d2 - (b * d2 - aa * oc2) * is) * ia;
-          gr = -rr * is;
-        } else {
-          gc0 = d0 * ia;
-          gc1 = d1 * ia;
-          gc2 = d2 * ia;
-          gr = 0.0;
-        }
-        double ld = (double)__ldg(a.dl_ddepth + p);
+        const int local = (int)(p - a.pix_base[v]);  // a view has fewer than 2^31 pixels
+        const Ray r = make_ray(V.m, V.width, V.height, V.pane, local % V.width, local / V.width);
+        entry_gradient(r, __ldg(a.pos + h), __ldg(a.radius + h), __ldg(a.dl_ddepth + p), g + 3);
         g[0] = __ldg(a.dl_drgb + 3 * p + 0);
         g[1] = __ldg(a.dl_drgb + 3 * p + 1);
         g[2] = __ldg(a.dl_drgb + 3 * p + 2);
-        g[3] = (float)(ld * gc0);
-        g[4] = (float)(ld * gc1);
-        g[5] = (float)(ld * gc2);
-        g[6] = (float)(ld * gr);
       }
     }
-    unsigned peers = __match_any_sync(FULL, h);
-    int leader = __ffs(peers) - 1;
-    float sum[7];
+    // sums over runs of equal hits, in the run's first lane
+    const int lane = threadIdx.x & 31;
+    const int32_t before = __shfl_up_sync(FULL, h, 1);
+    const unsigned heads = __ballot_sync(FULL, lane == 0 || h != before);
+    const unsigned above = heads >> lane >> 1;
+    const int last = above ? lane + __ffs(above) - 1 : 31;  // of the lane's run
+    const int longest = __reduce_max_sync(FULL, last - lane);
+    for (int off = 1; off <= longest; off *= 2) {
 #pragma unroll
-    for (int k = 0; k < 7; ++k) sum[k] = 0.0f;
-    // every lane of the group walks the same peer list, so the masked shuffles line up
-    unsigned m = peers;
-    while (m) {
-      int src = __ffs(m) - 1;
-#pragma unroll
-      for (int k = 0; k < 7; ++k) sum[k] += __shfl_sync(peers, g[k], src);
-      m &= m - 1;
+      for (int k = 0; k < 7; ++k) {
+        const float o = __shfl_down_sync(FULL, g[k], off);
+        if (lane + off <= last) g[k] += o;
+      }
     }
-    if (h >= 0 && (int)(threadIdx.x & 31) == leader) {
-      atomicAdd(a.g_rgb + 3 * (int64_t)h + 0, sum[0]);
-      atomicAdd(a.g_rgb + 3 * (int64_t)h + 1, sum[1]);
-      atomicAdd(a.g_rgb + 3 * (int64_t)h + 2, sum[2]);
-      atomicAdd(a.g_xyz + 3 * (int64_t)h + 0, sum[3]);
-      atomicAdd(a.g_xyz + 3 * (int64_t)h + 1, sum[4]);
-      atomicAdd(a.g_xyz + 3 * (int64_t)h + 2, sum[5]);
-      atomicAdd(a.g_radius + h, sum[6]);
+    if (h >= 0 && ((heads >> lane) & 1u)) {
+      atomicAdd(a.g_rgb + 3 * (int64_t)h + 0, g[0]);
+      atomicAdd(a.g_rgb + 3 * (int64_t)h + 1, g[1]);
+      atomicAdd(a.g_rgb + 3 * (int64_t)h + 2, g[2]);
+      atomicAdd(a.g_xyz + 3 * (int64_t)h + 0, g[3]);
+      atomicAdd(a.g_xyz + 3 * (int64_t)h + 1, g[4]);
+      atomicAdd(a.g_xyz + 3 * (int64_t)h + 2, g[5]);
+      atomicAdd(a.g_radius + h, g[6]);
     }
   }
 }
