@@ -178,10 +178,7 @@ __device__ __forceinline__ void klist_insert(KList<K>& L, float d, int32_t s, fl
 // compare-and-swap chain would leave the warp waiting on each result).
 // Exact d2 ties only matter when one of the tied entries is about to leave
 // the set; that case (the 9th and 10th entries equal) takes the ordered
-// path, which compares cloud indices.  An earlier form kept the previous
-// step's points in the set and re-sorted them; the walk then met each of
-// them a second time, and every insertion had to test for duplicates first
-// (that form was 6% slower, with 80 more bytes of spills at 64 registers).
+// path, which compares cloud indices.
 struct KSet {
   float d[KNN];
   int32_t s[KNN];   // sorted position, -1 = empty
@@ -214,51 +211,75 @@ struct KSet {
       s[0] = g0 ? ss : s[0];
       return;
     }
-    order(perm);
-    consider_ordered(dd, ss, perm);
+    float td[KNN];
+    int32_t ts[KNN];
+    spill(td, ts);
+    consider_ordered(td, ts, dd, ss, perm);
+    fill(td, ts);
   }
 
-  // Equal distances present: skip a duplicate, else insert by (d2, cloud index).
-  __device__ __forceinline__ void consider_ordered(float dd, int32_t ss, const int32_t* __restrict__ perm) {
-    bool dup = false;
-#pragma unroll
-    for (int j = 0; j < KNN; ++j) dup |= (s[j] == ss);
-    if (dup) return;
-#pragma unroll
-    for (int j = 0; j < KNN; ++j) {
-      if (s[j] < 0 || knn_before(dd, ss, d[j], s[j], perm)) {  // placeholders are last
-        const float td = d[j];
-        const int32_t ts = s[j];
-        d[j] = dd;
-        s[j] = ss;
-        dd = td;
-        ss = ts;
-      }
-    }
-  }
-
-  // Sorts runs of equal d2 by cloud index (an insertion pass, taken only
-  // when two adjacent real entries have equal d2).
+  // Sorts runs of equal d2 by cloud index.
   __device__ __forceinline__ void order(const int32_t* __restrict__ perm) {
     bool tie = false;
 #pragma unroll
     for (int j = 0; j + 1 < KNN; ++j) tie |= (d[j] == d[j + 1] && s[j + 1] >= 0);
     if (tie) {
-#pragma unroll
-      for (int i = 1; i < KNN; ++i) {
-#pragma unroll
-        for (int j = i; j > 0; --j) {
-          if (s[j] >= 0 && knn_before(d[j], s[j], d[j - 1], s[j - 1], perm)) {
-            const float td = d[j];
-            const int32_t ts = s[j];
-            d[j] = d[j - 1];
-            s[j] = s[j - 1];
-            d[j - 1] = td;
-            s[j - 1] = ts;
-          }
-        }
-      }
+      float td[KNN];
+      int32_t ts[KNN];
+      spill(td, ts);
+      order_ties(td, ts, perm);
+      fill(td, ts);
     }
+  }
+
+  // The paths for exact ties work on a copy in local memory, in rolled loops:
+  // they are next to never taken, and unrolled over registers they were most
+  // of the kernel's code, spread between the instructions of the walk (the
+  // marcher lost 15% to instruction fetch).
+  __device__ __forceinline__ void spill(float* td, int32_t* ts) const {
+#pragma unroll
+    for (int j = 0; j < KNN; ++j) {
+      td[j] = d[j];
+      ts[j] = s[j];
+    }
+  }
+  __device__ __forceinline__ void fill(const float* td, const int32_t* ts) {
+#pragma unroll
+    for (int j = 0; j < KNN; ++j) {
+      d[j] = td[j];
+      s[j] = ts[j];
+    }
+  }
+  static __device__ __forceinline__ void order_ties(float* td, int32_t* ts, const int32_t* __restrict__ perm) {
+#pragma unroll 1
+    for (int i = 1; i < KNN; ++i)
+#pragma unroll 1
+      for (int j = i; j > 0 && ts[j] >= 0 && knn_before(td[j], ts[j], td[j - 1], ts[j - 1], perm); --j) {
+        const float a = td[j];
+        td[j] = td[j - 1];
+        td[j - 1] = a;
+        const int32_t b = ts[j];
+        ts[j] = ts[j - 1];
+        ts[j - 1] = b;
+      }
+  }
+  // Equal distances present: skip a duplicate, else insert by (d2, cloud index).
+  static __device__ __forceinline__ void consider_ordered(float* td, int32_t* ts, float dd, int32_t ss,
+                                                          const int32_t* __restrict__ perm) {
+    order_ties(td, ts, perm);
+#pragma unroll 1
+    for (int j = 0; j < KNN; ++j)
+      if (ts[j] == ss) return;
+#pragma unroll 1
+    for (int j = 0; j < KNN; ++j)
+      if (ts[j] < 0 || knn_before(dd, ss, td[j], ts[j], perm)) {  // placeholders are last
+        const float a = td[j];
+        td[j] = dd;
+        dd = a;
+        const int32_t b = ts[j];
+        ts[j] = ss;
+        ss = b;
+      }
   }
 
   // Start of a step.  The previous step's ten points, re-measured at the new
@@ -287,21 +308,16 @@ struct KSet {
   }
 
   // src/ray_marching.cu:280-290: min of sqrtf(d2) - r visiting candidates
-  // in ascending (d2, index) order with a strict "<" -- equivalently the
-  // minimum value, ties going to the smaller (d2, index).
+  // in ascending (d2, index) order with a strict "<" (after order()).
   __device__ __forceinline__ float step_value(const IndexDev& ix, int32_t* best_s) const {
-    float best = __int_as_float(0x7f800000), bd = best;
+    float best = __int_as_float(0x7f800000);
     int32_t bs = -1;
 #pragma unroll
     for (int j = 0; j < KNN; ++j) {
       if (s[j] >= 0) {
         float v = __fsub_rn(__fsqrt_rn(d[j]), __ldg(&ix.rec[s[j]].w));
-        bool take = v < best;
-        if (!take && v == best)
-          take = d[j] < bd || (d[j] == bd && __ldg(ix.perm + s[j]) < __ldg(ix.perm + bs));
-        if (take) {
+        if (v < best) {
           best = v;
-          bd = d[j];
           bs = s[j];
         }
       }
@@ -640,7 +656,7 @@ constexpr int PKT_OVERFLOW = 256;
 struct PacketQueue {
   union {
     struct {
-      float4 rec[32];  // one staged leaf (leaf size <= 32)
+      alignas(16) float x[32], y[32], z[32];  // one staged leaf (leaf size <= 32)
       uint32_t code[PSTACK];
       uint32_t over[PKT_OVERFLOW];
     };
@@ -650,11 +666,6 @@ struct PacketQueue {
   unsigned n_dfs;
 };
 
-__device__ __forceinline__ void list_consider_unique(KSet& L, float d, int32_t s, float r,
-                                                     const int32_t* perm) {
-  (void)r;
-  L.consider(d, s, perm);
-}
 #define RM_CSWAP_U(ka, ca, kb, cb)                 \
   do {                                             \
     if ((kb) < (ka)) {                             \
@@ -829,7 +840,7 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
       }
       if (lvl + 1 == ix.depth) {
         const uint32_t lbase = (G - last_first) * 4u;
-#pragma unroll
+#pragma unroll 1  // one copy of the scan: four cost more in instruction fetch
         for (int t = 0; t < 4; ++t) {
           const int c = (int)((order >> (2 * t)) & 3u);
           if (!(needm & (1u << c))) continue;
@@ -839,28 +850,39 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
           const int64_t start = (int64_t)(lbase + c) * ix.leaf;
           const int cnt = (int)min((int64_t)ix.leaf, ix.n - start);
           ++leaves;
-          // one coalesced load of the leaf into shared memory, then broadcast
-          // reads, two points per iteration: their distances are independent
-          // (twice the work between dependent instructions), while the
-          // insertion stays inlined at one site, in a two-pass loop that only
-          // runs when one of the two is within the bound (unrolling the
-          // insertion as well costs more in instruction fetch than it saves;
-          // two points per iteration measured +2.8%)
+          // The leaf goes to shared memory as coordinate arrays; lanes then
+          // read four points at a time and measure them with paired
+          // arithmetic (the same bits as d2_point): 15 instructions for four
+          // distances instead of 28, 256 -> 242 ms for 24 views at 20M
+          // points.  Slots past the leaf's end hold NaN, which is within no
+          // bound.
           __syncwarp();
-          if (lane < cnt) ps.rec[lane] = __ldg(ix.rec + start + lane);
+          {
+            const float none = __int_as_float(0x7fffffff);
+            const float4 c = lane < cnt ? __ldg(ix.rec + start + lane) : make_float4(none, none, none, 0.0f);
+            ps.x[lane] = c.x;
+            ps.y[lane] = c.y;
+            ps.z[lane] = c.z;
+          }
           __syncwarp();
           if (active) {
-            for (int k = 0; k < cnt; k += 2) {
-              const float4 ca = ps.rec[k], cb = ps.rec[k + 1];  // rec has 32 slots; cb unused past cnt
-              const float da = d2_point(ca, qx, qy, qz);
-              const float db = k + 1 < cnt ? d2_point(cb, qx, qy, qz) : INF;
-              if (fminf(da, db) <= list_worst(L)) {
-#pragma unroll 1
-                for (int j = 0; j < 2; ++j) {
-                  const float dj = j ? db : da;
-                  if (dj <= list_worst(L)) list_consider_unique(L, dj, (int32_t)(start + k + j), 0.0f, ix.perm);
-                }
+            for (int k = 0; k < cnt; k += 4) {
+              float d0, d1, d2, d3;
+              {
+                const float4 X = *reinterpret_cast<const float4*>(ps.x + k);
+                const float4 Y = *reinterpret_cast<const float4*>(ps.y + k);
+                const float4 Z = *reinterpret_cast<const float4*>(ps.z + k);
+                const unsigned long long x0 = f2_sub(f2_pack(X.x, X.y), qx2), x1 = f2_sub(f2_pack(X.z, X.w), qx2);
+                const unsigned long long y0 = f2_sub(f2_pack(Y.x, Y.y), qy2), y1 = f2_sub(f2_pack(Y.z, Y.w), qy2);
+                const unsigned long long z0 = f2_sub(f2_pack(Z.x, Z.y), qz2), z1 = f2_sub(f2_pack(Z.z, Z.w), qz2);
+                f2_unpack(f2_fma(z0, z0, f2_fma(x0, x0, f2_mul(y0, y0))), d0, d1);
+                f2_unpack(f2_fma(z1, z1, f2_fma(x1, x1, f2_mul(y1, y1))), d2, d3);
               }
+              const int32_t s = (int32_t)start + k;
+              if (d0 <= list_worst(L)) list_consider(L, d0, s, 0.0f, ix.perm);
+              if (d1 <= list_worst(L)) list_consider(L, d1, s + 1, 0.0f, ix.perm);
+              if (d2 <= list_worst(L)) list_consider(L, d2, s + 2, 0.0f, ix.perm);
+              if (d3 <= list_worst(L)) list_consider(L, d3, s + 3, 0.0f, ix.perm);
             }
           }
         }
