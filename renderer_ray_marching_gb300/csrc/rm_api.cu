@@ -74,6 +74,11 @@ const void* stage_in(Ctx& c, DevBuf& buf, const void* src, size_t bytes, int loc
   return buf.p;
 }
 
+void throw_kernel_errors(unsigned long long count) {
+  if (count)
+    throw KernelError("kernel reported " + std::to_string(count) + " incomplete nearest-neighbour searches");
+}
+
 // Error slots: the radii/kNN kernels count failed searches at err_counter,
 // the marchers at counters[3] (stack bound or node budget exceeded).
 void check_kernel_errors(Ctx& c) {
@@ -81,8 +86,7 @@ void check_kernel_errors(Ctx& c) {
   CK(cudaMemcpyAsync(&e[0], err_counter(c), sizeof(e[0]), cudaMemcpyDeviceToHost, c.stream));
   CK(cudaMemcpyAsync(&e[1], counters(c) + 3, sizeof(e[1]), cudaMemcpyDeviceToHost, c.stream));
   CK(cudaStreamSynchronize(c.stream));
-  if (e[0] || e[1])
-    throw KernelError("kernel reported " + std::to_string(e[0] + e[1]) + " incomplete nearest-neighbour searches");
+  throw_kernel_errors(e[0] + e[1]);
 }
 
 bool view_ok(const rm_view& v, std::string* why) {
@@ -203,8 +207,8 @@ void rm_ctx_destroy(rm_ctx* ctx) {
   if (c.stream) cudaStreamSynchronize(c.stream);
   c.drop_graph();
   DevBuf* bufs[] = {&c.pos, &c.radii_clamped, &c.rec, &c.col, &c.perm, &c.groups,
-                    &c.keys[0], &c.keys[1], &c.vals[0], &c.vals[1], &c.sort_counts,
-                    &c.scan_sums, &c.scratch_bounds, &c.scalars, &c.staging_in, &c.staging_out,
+                    &c.keys, &c.vals, &c.sort_counts,
+                    &c.scan_sums, &c.scratch_bounds, &c.bucket_i, &c.scalars, &c.staging_in, &c.staging_out,
                     &c.views, &c.frame_bufs, &c.queue, &c.tail};
   for (DevBuf* b : bufs) b->release();
   if (c.pinned_views) cudaFreeHost(c.pinned_views);
@@ -329,8 +333,12 @@ rm_status rm_radii_compute(rm_ctx* ctx, float max_radius, float* radii_out, int3
     CK(cudaMemsetAsync(err_counter(c), 0, 8, c.stream));
     launch_radii(c, max_radius, dr, dn);  // also sets the records' radii
     CK(cudaGetLastError());
-    refresh_max_radius(c);
-    check_kernel_errors(c);
+    // the largest radius and the error counts in one read
+    unsigned long long sc[32];
+    CK(cudaMemcpyAsync(sc, c.scalars.p, sizeof(sc), cudaMemcpyDeviceToHost, c.stream));
+    CK(cudaStreamSynchronize(c.stream));
+    set_max_radius(c, (unsigned)sc[4]);
+    throw_kernel_errors(sc[8] + sc[16 + 3]);
     if (loc == RM_HOST) {
       if (radii_out) CK(cudaMemcpyAsync(radii_out, dr, n * 4, cudaMemcpyDeviceToHost, c.stream));
       if (nn_out) CK(cudaMemcpyAsync(nn_out, dn, n * 4, cudaMemcpyDeviceToHost, c.stream));

@@ -6,7 +6,7 @@
 //   1. bounds:   block-reduced min/max of the cloud (+ a non-finite flag);
 //   2. keys:     32-bit Hilbert-curve key of each point's cubic cell;
 //   3. sort:     LSD radix sort of (key, cloud index), 4 passes of 8 bits,
-//                stable warp-level ranking with __match_any_sync;
+//                stable warp-level ranking by digit votes;
 //   4. blocks:   1024 consecutive points per CTA, split by medians down to
 //                leaves of `leaf` points; packed float4 records (x, y, z,
 //                radius), colours and cloud indices in that order, and the
@@ -21,6 +21,7 @@
 // (d2, cloud index) ordering, so only speed depends on the layout.
 #include "rm_internal.h"
 
+#include <algorithm>
 #include <cstring>
 
 namespace rm {
@@ -86,16 +87,22 @@ __global__ void k_bounds_partial(const float4* __restrict__ pos, int64_t n,
   }
 }
 
+// Warp a reduces component a of the partials.
 __global__ void k_bounds_final(const float* __restrict__ part, int nblocks,
                                float* __restrict__ out) {
-  int a = threadIdx.x;
+  const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (a >= 7) return;
   float v = part[a];
-  for (int b = 1; b < nblocks; ++b) {
-    float x = part[b * 8 + a];
+  for (int b = lane; b < nblocks; b += 32) {
+    const float x = part[b * 8 + a];
     v = (a < 3) ? fminf(v, x) : fmaxf(v, x);
   }
-  out[a] = v;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) {
+    const float x = __shfl_xor_sync(0xffffffffu, v, off);
+    v = (a < 3) ? fminf(v, x) : fmaxf(v, x);
+  }
+  if (lane == 0) out[a] = v;
 }
 
 // ---------------------------------------------------------------- curve keys
@@ -186,8 +193,7 @@ __global__ void k_coarse_count(const float4* __restrict__ pos, int64_t n, const 
 // of the points of the cell beyond a near face (at most a quarter cell away)
 // takes its key from that cell's edge.
 __global__ void k_curve_keys(const float4* __restrict__ pos, int64_t n, const float* __restrict__ bounds, int g,
-                             const uint32_t* __restrict__ count, uint32_t* __restrict__ keys,
-                             uint32_t* __restrict__ vals) {
+                             const uint32_t* __restrict__ count, uint32_t* __restrict__ keys) {
   const CurveGrid grid(bounds);
   const int sh = CURVE_BITS - g;
   const uint32_t quarter = 1u << sh >> 2, in = (1u << sh) - 1u;
@@ -216,7 +222,6 @@ __global__ void k_curve_keys(const float4* __restrict__ pos, int64_t n, const fl
     for (int a = 0; a < 3; ++a)
       if (axis == a) q[a] = to;
     keys[i] = curve_key(q[0], q[1], q[2]);
-    vals[i] = (uint32_t)i;
   }
 }
 
@@ -224,6 +229,14 @@ __global__ void k_curve_keys(const float4* __restrict__ pos, int64_t n, const fl
 // Tile = SORT_THREADS threads x SORT_ITEMS keys; warp w owns the contiguous
 // run [w*32*SORT_ITEMS, (w+1)*32*SORT_ITEMS) of its tile, processed in
 // rounds of 32 consecutive keys, so ranks follow input order (stable).
+//
+// Bound by HBM: a pass reads and writes 16 bytes per point (and its counts
+// read 4).  A tile is put in digit order in shared memory first and goes out
+// in runs of one digit, so that stores fill whole sectors; written from
+// registers in input order a pass took 0.30 ms at 20M points and 2.3 ms at
+// 100M, now 0.11 and 0.49 (3.3 TB/s).  Tiles of 8192 measured 0.52 ms at 100M,
+// votes of __match_any_sync instead of one per bit 0.60.  The first pass
+// takes each key's index from its position.
 constexpr int SORT_THREADS = 256;
 constexpr int SORT_ITEMS = 16;
 constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;
@@ -236,10 +249,22 @@ k_sort_hist(const uint32_t* __restrict__ keys, int64_t n, int shift, int64_t nti
   __shared__ uint32_t hist[RADIX];
   for (int d = threadIdx.x; d < RADIX; d += blockDim.x) hist[d] = 0;
   __syncthreads();
-  int64_t base = (int64_t)blockIdx.x * SORT_TILE;
-  for (int k = threadIdx.x; k < SORT_TILE; k += SORT_THREADS) {
-    int64_t i = base + k;
-    if (i < n) atomicAdd(&hist[(keys[i] >> shift) & (RADIX - 1)], 1u);
+  const int64_t base = (int64_t)blockIdx.x * SORT_TILE;
+  if (base + SORT_TILE <= n) {
+    const uint4* k4 = reinterpret_cast<const uint4*>(keys + base);  // tiles start on 32 KB
+    uint4 v[SORT_ITEMS / 4];
+#pragma unroll
+    for (int r = 0; r < SORT_ITEMS / 4; ++r) v[r] = __ldg(k4 + r * SORT_THREADS + threadIdx.x);
+#pragma unroll
+    for (int r = 0; r < SORT_ITEMS / 4; ++r) {
+      atomicAdd(&hist[(v[r].x >> shift) & (RADIX - 1)], 1u);
+      atomicAdd(&hist[(v[r].y >> shift) & (RADIX - 1)], 1u);
+      atomicAdd(&hist[(v[r].z >> shift) & (RADIX - 1)], 1u);
+      atomicAdd(&hist[(v[r].w >> shift) & (RADIX - 1)], 1u);
+    }
+  } else {
+    for (int64_t i = base + threadIdx.x; i < n; i += SORT_THREADS)
+      atomicAdd(&hist[(keys[i] >> shift) & (RADIX - 1)], 1u);
   }
   __syncthreads();
   for (int d = threadIdx.x; d < RADIX; d += blockDim.x)
@@ -324,57 +349,103 @@ k_scan_add(uint32_t* __restrict__ data, int64_t len, const uint32_t* __restrict_
   }
 }
 
-__global__ void __launch_bounds__(SORT_THREADS)
+// Exclusive prefix over RADIX digit counts held by the first RADIX threads;
+// all threads of the block call it.
+__device__ __forceinline__ uint32_t digit_prefix(uint32_t v, uint32_t* warp_sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+    if (lane >= off) x += y;
+  }
+  if (lane == 31 && warp < RADIX / 32) warp_sums[warp] = x;
+  __syncthreads();
+  uint32_t before = 0;
+  for (int w = 0; w < warp && w < RADIX / 32; ++w) before += warp_sums[w];
+  return before + x - v;
+}
+
+struct SortSmem {
+  uint32_t cnt[SORT_WARPS][RADIX];  // per warp: keys of each digit, then the warp's first place
+  uint32_t base[RADIX];             // global place of the tile's first key of a digit, less its local place
+  uint32_t sums[RADIX / 32];
+  uint32_t key[SORT_TILE], val[SORT_TILE];
+};
+
+template <bool FIRST>
+__global__ void __launch_bounds__(SORT_THREADS, 4)
 k_sort_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                int64_t n, int shift, int64_t ntiles, const uint32_t* __restrict__ offsets,
                uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out) {
-  __shared__ uint32_t wcnt[SORT_WARPS][RADIX];
-  __shared__ uint32_t gbase[RADIX];
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int d = lane; d < RADIX; d += 32) wcnt[warp][d] = 0;
-  for (int d = threadIdx.x; d < RADIX; d += SORT_THREADS)
-    gbase[d] = offsets[(int64_t)d * ntiles + blockIdx.x];
-  __syncthreads();
+  extern __shared__ __align__(16) unsigned char sort_smem[];
+  SortSmem& sm = *reinterpret_cast<SortSmem*>(sort_smem);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int d = lane; d < RADIX; d += 32) sm.cnt[warp][d] = 0;
+  __syncwarp();
   const uint32_t lt_mask = (1u << lane) - 1u;
-  int64_t wbase = (int64_t)blockIdx.x * SORT_TILE + (int64_t)warp * 32 * SORT_ITEMS;
-  uint32_t key[SORT_ITEMS], val[SORT_ITEMS], rank[SORT_ITEMS];
+  const int64_t tile = (int64_t)blockIdx.x * SORT_TILE;
+  const int64_t wbase = tile + (int64_t)warp * 32 * SORT_ITEMS;
+  uint32_t key[SORT_ITEMS], rank[SORT_ITEMS / 2];  // ranks in 16 bits
 #pragma unroll
   for (int r = 0; r < SORT_ITEMS; ++r) {
-    int64_t i = wbase + r * 32 + lane;
-    bool valid = i < n;
-    key[r] = valid ? keys_in[i] : 0u;
-    val[r] = valid ? vals_in[i] : 0u;
-    // invalid lanes use a private digit value RADIX that matches no real digit
-    uint32_t dig = valid ? ((key[r] >> shift) & (RADIX - 1)) : (uint32_t)RADIX;
-    uint32_t peers = __match_any_sync(0xffffffffu, dig);
-    uint32_t before = __popc(peers & lt_mask);
-    uint32_t prev = valid ? wcnt[warp][dig] : 0u;
+    const int64_t i = wbase + r * 32 + lane;
+    key[r] = i < n ? __ldcs(keys_in + i) : 0u;
+  }
+#pragma unroll
+  for (int r = 0; r < SORT_ITEMS; ++r) {
+    const bool valid = wbase + r * 32 + lane < n;
+    const uint32_t dig = (key[r] >> shift) & (RADIX - 1);
+    // lanes with the same digit, one vote per bit
+    uint32_t peers = __ballot_sync(0xffffffffu, valid);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const uint32_t v = __ballot_sync(0xffffffffu, (dig >> b) & 1u);
+      peers &= (dig >> b) & 1u ? v : ~v;
+    }
+    const uint32_t before = __popc(peers & lt_mask);
+    const uint32_t prev = valid ? sm.cnt[warp][dig] : 0u;
     __syncwarp();
-    if (valid && before == 0) wcnt[warp][dig] = prev + __popc(peers);
+    if (valid && before == 0) sm.cnt[warp][dig] = prev + __popc(peers);
     __syncwarp();
-    rank[r] = prev + before;
+    if (r & 1) rank[r / 2] |= (prev + before) << 16;
+    else rank[r / 2] = prev + before;
   }
   __syncthreads();
-  // per digit: exclusive prefix over warps
-  for (int d = threadIdx.x; d < RADIX; d += SORT_THREADS) {
-    uint32_t run = 0;
+  // places within the tile: digits in order, and within a digit the warps
+  uint32_t total = 0;
+  const int d = threadIdx.x;
+  if (d < RADIX)
+#pragma unroll
+    for (int w = 0; w < SORT_WARPS; ++w) total += sm.cnt[w][d];
+  const uint32_t first = digit_prefix(d < RADIX ? total : 0u, sm.sums);
+  if (d < RADIX) {
+    sm.base[d] = offsets[(int64_t)d * ntiles + blockIdx.x] - first;
+    uint32_t run = first;
 #pragma unroll
     for (int w = 0; w < SORT_WARPS; ++w) {
-      uint32_t c = wcnt[w][d];
-      wcnt[w][d] = run;
+      const uint32_t c = sm.cnt[w][d];
+      sm.cnt[w][d] = run;
       run += c;
     }
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < SORT_ITEMS; ++r) {
-    int64_t i = wbase + r * 32 + lane;
+    const int64_t i = wbase + r * 32 + lane;
     if (i < n) {
-      uint32_t dig = (key[r] >> shift) & (RADIX - 1);
-      uint32_t dst = gbase[dig] + wcnt[warp][dig] + rank[r];
-      keys_out[dst] = key[r];
-      vals_out[dst] = val[r];
+      const uint32_t at = sm.cnt[warp][(key[r] >> shift) & (RADIX - 1)] + (r & 1 ? rank[r / 2] >> 16 : rank[r / 2] & 0xffffu);
+      sm.key[at] = key[r];
+      sm.val[at] = FIRST ? (uint32_t)i : __ldcs(vals_in + i);
     }
+  }
+  __syncthreads();
+  const int m = (int)min((int64_t)SORT_TILE, n - tile);
+  for (int j = threadIdx.x; j < m; j += SORT_THREADS) {
+    const uint32_t k = sm.key[j];
+    const uint32_t dst = sm.base[(k >> shift) & (RADIX - 1)] + (uint32_t)j;
+    keys_out[dst] = k;
+    vals_out[dst] = sm.val[j];
   }
 }
 
@@ -726,16 +797,24 @@ void launch_clamp_radii(Ctx& c, const float* in, float max_radius) {
   refresh_max_radius(c);
 }
 
-void refresh_max_radius(Ctx& c) {
+void launch_max_radius(Ctx& c) {
   unsigned int* mr = c.scalars.ptr<unsigned int>() + 8;
   CK(cudaMemsetAsync(mr, 0, sizeof(unsigned int), c.stream));
   k_max_radius<<<grid_for(c.n, 256, 1024), 256, 0, c.stream>>>(c.radii_clamped.ptr<float>(), c.n, mr);
-  unsigned int bits = 0;
-  CK(cudaMemcpyAsync(&bits, mr, sizeof(bits), cudaMemcpyDeviceToHost, c.stream));
-  CK(cudaStreamSynchronize(c.stream));
+}
+
+void set_max_radius(Ctx& c, unsigned bits) {
   float r;
   memcpy(&r, &bits, sizeof(r));
   c.max_r = (r < INFINITY) ? r : INFINITY;
+}
+
+void refresh_max_radius(Ctx& c) {
+  launch_max_radius(c);
+  unsigned int bits = 0;
+  CK(cudaMemcpyAsync(&bits, c.scalars.ptr<unsigned int>() + 8, sizeof(bits), cudaMemcpyDeviceToHost, c.stream));
+  CK(cudaStreamSynchronize(c.stream));
+  set_max_radius(c, bits);
 }
 
 // Builds the index from c.pos / c.rgb.  Returns false (with c.err set) on
@@ -747,7 +826,7 @@ bool build_index(Ctx& c) {
   int nb = grid_for(n, 256, 1024);
   c.scratch_bounds.reserve((size_t)nb * 8 * sizeof(float));
   k_bounds_partial<<<nb, 256, 0, st>>>(c.pos.ptr<float4>(), n, c.scratch_bounds.ptr<float>());
-  k_bounds_final<<<1, 32, 0, st>>>(c.scratch_bounds.ptr<float>(), nb, c.scalars.ptr<float>());
+  k_bounds_final<<<1, 7 * 32, 0, st>>>(c.scratch_bounds.ptr<float>(), nb, c.scalars.ptr<float>());
   float hb[8];
   CK(cudaMemcpyAsync(hb, c.scalars.ptr<float>(), 8 * sizeof(float), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
@@ -758,20 +837,18 @@ bool build_index(Ctx& c) {
   for (int a = 0; a < 6; ++a) c.bounds[a] = hb[a];
 
   // keys
-  c.keys[0].reserve((size_t)n * 4);
-  c.keys[1].reserve((size_t)n * 4);
-  c.vals[0].reserve((size_t)n * 4);
-  c.vals[1].reserve((size_t)n * 4);
   // Coarse cells of about 500 points where points lie on surfaces (about
   // 2.5 cells across occupied per cell of a face), half a block of the tree.
   int g = 1;
   while (g < 8 && n > (int64_t)1280 << (2 * g + 1)) ++g;
-  c.keys[1].reserve((size_t)4 << (3 * g));  // counted in the sort's second buffer
-  uint32_t* coarse = c.keys[1].ptr<uint32_t>();
+  c.half = std::max((n + 63) / 64 * 64, (int64_t)1 << (3 * g));  // halves start on 256 bytes
+  c.keys.reserve((size_t)c.half * 8);
+  c.vals.reserve((size_t)c.half * 8);
+  uint32_t* coarse = c.key(1);  // counted in the sort's second buffer
   CK(cudaMemsetAsync(coarse, 0, (size_t)4 << (3 * g), st));
   k_coarse_count<<<grid_for((n + 7) / 8, 256), 256, 0, st>>>(c.pos.ptr<float4>(), n, c.scalars.ptr<float>(), g, coarse);
   k_curve_keys<<<grid_for(n, 256), 256, 0, st>>>(c.pos.ptr<float4>(), n, c.scalars.ptr<float>(), g, coarse,
-                                                 c.keys[0].ptr<uint32_t>(), c.vals[0].ptr<uint32_t>());
+                                                 c.key(0));
   // radix sort, 32-bit keys: shifts 0, 8, 16, 24
   int64_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
   int64_t clen = ntiles * RADIX;
@@ -781,13 +858,18 @@ bool build_index(Ctx& c) {
   int cur = 0;
   for (int shift = 0; shift < 32; shift += 8) {
     uint32_t* cnt = c.sort_counts.ptr<uint32_t>();
-    k_sort_hist<<<(unsigned)ntiles, SORT_THREADS, 0, st>>>(c.keys[cur].ptr<uint32_t>(), n, shift, ntiles, cnt);
+    k_sort_hist<<<(unsigned)ntiles, SORT_THREADS, 0, st>>>(c.key(cur), n, shift, ntiles, cnt);
     k_scan_tiles<<<(unsigned)nscan, SCAN_THREADS, 0, st>>>(cnt, clen, c.scan_sums.ptr<uint32_t>());
     k_scan_sums<<<1, SCAN_THREADS, 0, st>>>(c.scan_sums.ptr<uint32_t>(), nscan);
     k_scan_add<<<(unsigned)nscan, SCAN_THREADS, 0, st>>>(cnt, clen, c.scan_sums.ptr<uint32_t>());
-    k_sort_scatter<<<(unsigned)ntiles, SORT_THREADS, 0, st>>>(
-        c.keys[cur].ptr<uint32_t>(), c.vals[cur].ptr<uint32_t>(), n, shift, ntiles, cnt,
-        c.keys[cur ^ 1].ptr<uint32_t>(), c.vals[cur ^ 1].ptr<uint32_t>());
+    auto scatter = [&](auto kern) {
+      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem)));
+      kern<<<(unsigned)ntiles, SORT_THREADS, sizeof(SortSmem), st>>>(
+          c.key(cur), c.val(cur), n, shift, ntiles, cnt,
+          c.key(cur ^ 1), c.val(cur ^ 1));
+    };
+    if (shift == 0) scatter(k_sort_scatter<true>);
+    else scatter(k_sort_scatter<false>);
     cur ^= 1;
   }
   // leaves and tree
@@ -809,7 +891,7 @@ bool build_index(Ctx& c) {
   const unsigned nblocks = (unsigned)((n + BLK - 1) / BLK + 3) / 4 * 4;
   auto blocks = [&](auto kern) {
     kern<<<nblocks, BLK_THREADS, 0, st>>>(c.pos.ptr<float4>(), c.have_radii ? c.radii_clamped.ptr<float>() : nullptr,
-                                          c.vals[cur].ptr<uint32_t>(), n, depth, c.rec.ptr<float4>(),
+                                          c.val(cur), n, depth, c.rec.ptr<float4>(),
                                           c.col.ptr<uint32_t>(), c.perm.ptr<int32_t>(), c.groups.ptr<float4>());
   };
   if (leaf == 8) blocks(k_blocks<8>);

@@ -95,8 +95,14 @@ struct Ctx {
   DevBuf col;            // uint32 sorted, packed rgb
   DevBuf perm;           // int32, sorted position -> cloud index
   DevBuf groups;         // float4 child groups
-  DevBuf keys[2], vals[2];
+  // the sort's double buffers, two halves of `half` words each; the radii
+  // pass through them on their way to cloud order
+  DevBuf keys, vals;
+  int64_t half = 0;
+  uint32_t* key(int i) const { return keys.ptr<uint32_t>() + i * half; }
+  uint32_t* val(int i) const { return vals.ptr<uint32_t>() + i * half; }
   DevBuf sort_counts, scan_sums, scratch_bounds;
+  DevBuf bucket_i;       // cloud indices of radii on their way to cloud order
   DevBuf scalars;        // [0..6] bounds + flag, [8] max radius bits, [16..] counters
   DevBuf staging_in, staging_out;
   DevBuf views;          // ViewDev table
@@ -143,6 +149,8 @@ void launch_pack(Ctx& c, const float* xyz, int stride, const uint8_t* rgb, int64
 void launch_clamp_radii(Ctx& c, const float* in, float max_radius);
 void launch_clamp_radii_only(Ctx& c, const float* in, float max_radius);
 void launch_set_radius(Ctx& c);
+void launch_max_radius(Ctx& c);  // into scalars [8]
+void set_max_radius(Ctx& c, unsigned bits);
 void refresh_max_radius(Ctx& c);
 bool build_index(Ctx& c);
 

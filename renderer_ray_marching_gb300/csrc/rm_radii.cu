@@ -10,6 +10,8 @@
 // short passes write the results in cloud order and clamp.
 #include "rm_internal.h"
 
+#include <algorithm>
+
 namespace rm {
 
 __global__ void __launch_bounds__(128)
@@ -380,33 +382,141 @@ k_radii_hard(IndexDev ix, HardList hard, float* __restrict__ r_sorted, int32_t* 
   }
 }
 
-// Sorted-order radii to cloud order (main.cu:110-113 leaves them in PLY
-// order), one output array per launch.  Each launch reads its sorted input
-// and perm once, streaming (evict-first), and scatters 4-byte values over
-// one array of 4 N bytes; at up to about 25M points that array fits in L2,
-// where the scattered stores merge into whole sectors before they reach
-// DRAM.  MODE 0: unclamped radius; 1: neighbour's cloud index; 2: radius
-// clamped to max_radius (main.cu:144-149) -- the context's render radii --
-// also written into the records' .w in sorted order.
-template <int MODE>
-__global__ void k_radii_to_cloud(const float* __restrict__ r_sorted, const int32_t* __restrict__ nn_sorted,
-                                 const int32_t* __restrict__ perm, int64_t n, float max_radius,
-                                 void* __restrict__ out, float4* __restrict__ rec) {
+// Sorted-order results to cloud order (main.cu:110-113 leaves them in PLY
+// order).  Scattered stores cost an L2 request per point and array whatever
+// their size, so radius and neighbour go as one 8-byte pair; k_split then
+// streams the pairs apart into the caller's arrays and the context's clamped
+// radii, and the records get theirs in sorted order.
+//
+// Direct form: one scattering pass.  While the pairs fit in L2 their sectors
+// fill up there.
+__device__ __forceinline__ float clamp_radius(float r, float max_radius) {  // main.cu:144-149
+  return (max_radius > 0.0f && r > max_radius) ? max_radius : r;
+}
+__device__ __forceinline__ void set_record(float4* __restrict__ rec, int64_t s, float r) {
+  float4 p = rec[s];  // whole records rewritten: full-sector stores
+  p.w = r;
+  rec[s] = p;
+}
+__global__ void k_to_cloud(const float* __restrict__ r_sorted, const int32_t* __restrict__ nn_sorted,
+                           const int32_t* __restrict__ perm, int64_t n, float max_radius, float4* __restrict__ rec,
+                           int2* __restrict__ pairs) {
   for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n; s += (int64_t)gridDim.x * blockDim.x) {
-    const int32_t i = __ldcs(perm + s);
-    if (MODE == 1) {
-      static_cast<int32_t*>(out)[i] = __ldcs(nn_sorted + s);
-    } else {
-      float r = __ldcs(r_sorted + s);
-      if (MODE == 2) {
-        r = (max_radius > 0.0f && r > max_radius) ? max_radius : r;
-        float4 c = rec[s];  // whole records rewritten: full-sector stores
-        c.w = r;
-        rec[s] = c;
-      }
-      static_cast<float*>(out)[i] = r;
-    }
+    const float r = __ldcs(r_sorted + s);
+    pairs[__ldcs(perm + s)] = make_int2(__float_as_int(r), __ldcs(nn_sorted + s));
+    set_record(rec, s, clamp_radius(r, max_radius));
   }
+}
+
+// Bucket form, for pairs beyond L2, where nearly every scattered store costs
+// a sector read and written in DRAM.  First the pairs are brought into
+// BUCKETS ranges of cloud indices: a tile is put in bucket order in shared
+// memory and goes out in runs, each tile taking its places in a bucket from
+// that bucket's cursor (the order inside a bucket does not matter).  A bucket
+// covers 2^shift cloud indices, exactly as many as it has places.  Then a
+// second pass scatters bucket by bucket, a few MB at a time.
+//
+// Bound by the scattered stores' L2 requests (95 G/s).  Direct and bucket
+// form without k_split: 53 and 87 us at 4M points, 131 and 182 at 8M, 643 and
+// 423 at 20M, 4.4 and 2.1 ms at 100M; three scattering passes of 4-byte
+// values took 0.70 ms at 20M and 11.0 ms at 100M where this, with k_split,
+// takes 0.49 and 2.4.
+constexpr int BUCKETS = 256;
+constexpr int BUCKET_THREADS = 256;
+constexpr int BUCKET_ITEMS = 16;
+constexpr int BUCKET_TILE = BUCKET_THREADS * BUCKET_ITEMS;
+constexpr int64_t BUCKET_MIN = 12 << 20;  // points from which the bucket form is taken
+struct BucketSmem {
+  uint32_t cnt[BUCKETS], first[BUCKETS], base[BUCKETS];
+  uint32_t sums[BUCKETS / 32];
+  int32_t i[BUCKET_TILE];
+  int2 pair[BUCKET_TILE];
+};
+__global__ void __launch_bounds__(BUCKET_THREADS, 4)
+k_to_buckets(const float* __restrict__ r_sorted, const int32_t* __restrict__ nn_sorted,
+             const int32_t* __restrict__ perm, int64_t n, int shift, float max_radius, float4* __restrict__ rec,
+             uint32_t* __restrict__ cursor, int32_t* __restrict__ to_i, int2* __restrict__ to_pair) {
+  extern __shared__ __align__(16) unsigned char bucket_smem[];
+  BucketSmem& sm = *reinterpret_cast<BucketSmem*>(bucket_smem);
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  sm.cnt[t] = 0;
+  __syncthreads();
+  const int64_t tile = (int64_t)blockIdx.x * BUCKET_TILE;
+  int32_t idx[BUCKET_ITEMS];
+  uint32_t rank[BUCKET_ITEMS];
+#pragma unroll
+  for (int k = 0; k < BUCKET_ITEMS; ++k) {
+    const int64_t s = tile + k * BUCKET_THREADS + t;
+    idx[k] = s < n ? __ldcs(perm + s) : -1;
+  }
+#pragma unroll
+  for (int k = 0; k < BUCKET_ITEMS; ++k)
+    if (idx[k] >= 0) rank[k] = atomicAdd(&sm.cnt[idx[k] >> shift], 1u);
+  __syncthreads();
+  const uint32_t c = sm.cnt[t];
+  uint32_t x = c;  // exclusive prefix over the buckets, one per thread
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
+    if (lane >= off) x += y;
+  }
+  if (lane == 31) sm.sums[warp] = x;
+  __syncthreads();
+  uint32_t first = x - c;
+  for (int w = 0; w < warp; ++w) first += sm.sums[w];
+  sm.first[t] = first;
+  sm.base[t] = c ? ((uint32_t)t << shift) + atomicAdd(cursor + t, c) - first : 0u;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < BUCKET_ITEMS; ++k) {
+    if (idx[k] < 0) continue;
+    const int64_t s = tile + k * BUCKET_THREADS + t;
+    const float r = __ldcs(r_sorted + s);
+    set_record(rec, s, clamp_radius(r, max_radius));
+    const uint32_t at = sm.first[idx[k] >> shift] + rank[k];
+    sm.i[at] = idx[k];
+    sm.pair[at] = make_int2(__float_as_int(r), __ldcs(nn_sorted + s));
+  }
+  __syncthreads();
+  const int count = (int)min((int64_t)BUCKET_TILE, n - tile);
+  for (int j = t; j < count; j += BUCKET_THREADS) {
+    const int32_t i = sm.i[j];
+    const uint32_t at = sm.base[i >> shift] + (uint32_t)j;
+    to_i[at] = i;
+    to_pair[at] = sm.pair[j];
+  }
+}
+// One tile per CTA, so that the resident CTAs work on adjacent tiles.
+__global__ void __launch_bounds__(BUCKET_THREADS)
+k_from_buckets(const int32_t* __restrict__ from_i, const int2* __restrict__ from_pair, int64_t n,
+               int2* __restrict__ pairs) {
+  const int64_t tile = (int64_t)blockIdx.x * BUCKET_TILE;
+#pragma unroll 8
+  for (int k = 0; k < BUCKET_ITEMS; ++k) {
+    const int64_t j = tile + k * BUCKET_THREADS + threadIdx.x;
+    if (j < n) pairs[__ldcs(from_i + j)] = __ldcs(from_pair + j);
+  }
+}
+
+// Pairs to the caller's arrays (either may be null) and the context's clamped
+// radii; `largest` gets the bits of the largest of those (they are >= 0).
+__global__ void k_split(const int2* __restrict__ pairs, int64_t n, float max_radius, float* __restrict__ radius,
+                        int32_t* __restrict__ nn, float* __restrict__ clamped, unsigned* __restrict__ largest) {
+  float m = 0.0f;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int2 p = __ldcs(pairs + i);
+    const float r = __int_as_float(p.x), c = clamp_radius(r, max_radius);
+    if (radius) radius[i] = r;
+    if (nn) nn[i] = p.y;
+    clamped[i] = c;
+    m = fmaxf(m, c);
+  }
+  __shared__ unsigned most;
+  if (threadIdx.x == 0) most = 0;
+  __syncthreads();
+  atomicMax(&most, __float_as_uint(m));
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(largest, most);
 }
 
 // General k-NN (k <= 32): one query per warp, the k nearest in the warp's
@@ -445,18 +555,19 @@ static int blocks_for(const Ctx& c, int64_t n, int threads) {
 }
 
 // Radii of every point: search, then cloud-order outputs, the context's
-// clamped radii and the records' radius lanes.
+// clamped radii, the records' radius lanes and the largest radius (on the
+// device, for read_max_radius).
 void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
   unsigned long long* err = c.scalars.ptr<unsigned long long>() + 8;
   if (c.launch.search == 1) {
     // sorted-order results in the radix sort's key buffers (N x 4 B each,
     // free once the index is built)
-    float* r_sorted = c.keys[0].ptr<float>();
-    int32_t* nn_sorted = c.keys[1].ptr<int32_t>();
+    float* r_sorted = reinterpret_cast<float*>(c.key(0));
+    int32_t* nn_sorted = reinterpret_cast<int32_t*>(c.key(1));
     unsigned long long* next = c.queue.ptr<unsigned long long>() + 1;
     // [1] region counter, [2] handed-over queries (positions in the sort's
     // value buffer, free like its key buffers)
-    const HardList hard{c.vals[0].ptr<uint32_t>(), next + 1};
+    const HardList hard{c.val(0), next + 1};
     CK(cudaMemsetAsync(next, 0, 2 * sizeof(unsigned long long), c.stream));
     auto go = [&](auto kern, int chunks) {
       int per_sm = 0;
@@ -470,18 +581,35 @@ void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
     if (c.n < RADII_SMALL) go(k_radii_region<1>, 1);
     else go(k_radii_region<2>, 2);
     k_radii_hard<<<(unsigned)(c.sm_count * 8), 32 * RADII_WARPS, 0, c.stream>>>(c.index(), hard, r_sorted, nn_sorted);
-    const int g = blocks_for(c, c.n, 256);
     const int32_t* perm = c.perm.ptr<int32_t>();
-    if (radii_out)
-      k_radii_to_cloud<0><<<g, 256, 0, c.stream>>>(r_sorted, nn_sorted, perm, c.n, max_radius, radii_out, nullptr);
-    if (nn_out)
-      k_radii_to_cloud<1><<<g, 256, 0, c.stream>>>(r_sorted, nn_sorted, perm, c.n, max_radius, nn_out, nullptr);
-    k_radii_to_cloud<2><<<g, 256, 0, c.stream>>>(r_sorted, nn_sorted, perm, c.n, max_radius,
-                                                 c.radii_clamped.ptr<float>(), c.rec.ptr<float4>());
+    float4* rec = c.rec.ptr<float4>();
+    int2* pairs = reinterpret_cast<int2*>(c.val(0));
+    if (c.n < BUCKET_MIN) {
+      k_to_cloud<<<blocks_for(c, c.n, 256), 256, 0, c.stream>>>(r_sorted, nn_sorted, perm, c.n, max_radius, rec, pairs);
+    } else {
+      int shift = 0;
+      while ((c.n - 1) >> shift >= BUCKETS) ++shift;
+      uint32_t* cursor = c.scratch_bounds.ptr<uint32_t>();
+      CK(cudaMemsetAsync(cursor, 0, BUCKETS * 4, c.stream));
+      c.bucket_i.reserve((size_t)c.n * 4);
+      int32_t* to_i = c.bucket_i.ptr<int32_t>();
+      CK(cudaFuncSetAttribute(k_to_buckets, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BucketSmem)));
+      const unsigned tiles = (unsigned)((c.n + BUCKET_TILE - 1) / BUCKET_TILE);
+      k_to_buckets<<<tiles, BUCKET_THREADS, sizeof(BucketSmem), c.stream>>>(r_sorted, nn_sorted, perm, c.n, shift,
+                                                                          max_radius, rec, cursor, to_i, pairs);
+      int2* apart = pairs;
+      pairs = reinterpret_cast<int2*>(c.key(0));  // the sorted results have been read
+      k_from_buckets<<<tiles, BUCKET_THREADS, 0, c.stream>>>(to_i, apart, c.n, pairs);
+    }
+    unsigned* largest = c.scalars.ptr<unsigned>() + 8;
+    CK(cudaMemsetAsync(largest, 0, sizeof(unsigned), c.stream));
+    k_split<<<std::min(blocks_for(c, c.n, 256), c.sm_count * 8), 256, 0, c.stream>>>(pairs, c.n, max_radius, radii_out, nn_out,
+                                                           c.radii_clamped.ptr<float>(), largest);
   } else {
     k_radii<<<blocks_for(c, c.n, 128), 128, 0, c.stream>>>(c.index(), max_radius, radii_out, nn_out,
                                                            c.radii_clamped.ptr<float>(), err);
     launch_set_radius(c);
+    launch_max_radius(c);
   }
 }
 

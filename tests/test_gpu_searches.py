@@ -54,8 +54,10 @@ def test_radii_and_knn(kind, n):
 
 
 @pytest.mark.parametrize("kind", ["room", "strays", "twins"])
-@pytest.mark.parametrize("n", [(5 << 20) - 1, (5 << 20) + 33])
-def test_radii_on_both_sides_of_the_region_switch(kind, n):
+@pytest.mark.parametrize("n", [(5 << 20) - 1, (5 << 20) + 33, (12 << 20) - 1, (12 << 20) + 4097])
+def test_radii_on_both_sides_of_the_size_switches(kind, n):
+    """Regions of one and two chunks; results to cloud order directly and
+    through buckets."""
     xyz = _cloud(kind, n)
     orad, onn = oracle.Index(xyz).radii(0.0)
     r = Renderer()
