@@ -52,13 +52,14 @@ k_radii(IndexDev ix, float max_radius, float* __restrict__ radii_out, int32_t* _
 // d2_box, and each gap is at most that of any query in the chunk, so a
 // needed leaf is never missed.
 //
-// Issue-bound (61% of the issue slots at 2M points).  One walk of the tree
+// Issue-bound (79% of the issue slots at 20M points).  One walk of the tree
 // per 32 queries, with every lane testing its own query against every box,
 // spent most of its instructions on the descent (59 expansions and 23 leaves
 // per warp in curve order).  Here an expansion tests 32 boxes at once, and
-// per chunk about 19 listed leaves are tested and 11 measured: 8.5 -> 3.7 ms
-// at 20M points, 61 -> 22 ms at 100M of uneven density, 76 -> 51 us at 100k
-// (together with the order of the records, k_blocks in rm_index.cu).
+// per chunk about 19 listed leaves are tested and 11 measured, four points at
+// a time (d2_point4: 3.6 -> 2.7 ms at 20M).  8.5 -> 2.9 ms at 20M points, 61 ->
+// 16 ms at 100M of uneven density, 76 -> 60 us at 100k, with the handed-over
+// queries and the order of the records (k_blocks in rm_index.cu).
 //
 // Memory traffic.  Warps take their regions from a global counter in sorted
 // order, so all resident warps work inside one window of a few MB that
@@ -66,32 +67,36 @@ k_radii(IndexDev ix, float max_radius, float* __restrict__ radii_out, int32_t* _
 // k_radii_to_cloud moves them to cloud order afterwards.
 constexpr int RADII_WARPS = 4;
 // Chunks per region.  Two share the descent, but make half as many, longer
-// regions: 1 against 2 chunks measured 0.33 / 0.40 ms for all of
-// rm_radii_compute at 1M points, 0.97 / 0.99 at 4M, 2.26 / 2.15 at 10M and
-// 15.0 / 13.8 at 50M (4 chunks: 0.50, 1.11, 2.36, 14.6).
-constexpr int64_t RADII_SMALL = 5 << 20;
+// regions: 1 against 2 chunks measured 0.12 / 0.19 ms at 500k points (search
+// and handed-over queries), 0.61 / 0.65 at 4M, 1.15 / 1.20 at 8M, 2.87 / 2.85
+// at 20M and 8.6 / 8.4 at 60M.
+constexpr int64_t RADII_SMALL = 12 << 20;
 constexpr int REGION_STACK = 512;  // depth-first, one node at a time, needs 3 entries per level beyond the last 64
 constexpr int REGION_LIST = 96;
-constexpr int REGION_SCANS = 3;  // scans of a full list, per chunk beyond the first, before a region gives up its walk
+// scans of a full list before a region gives up its walk
+template <int CHUNKS>
+constexpr int REGION_SCANS = CHUNKS == 1 ? 1 : 6;
 // In squared lengths, a chunk on a surface is about 55 times as wide as its
 // largest search; well above that its box says little (REGION_WIDE).  The
 // squared distances to the nearest neighbour on an even surface are
-// exponentially distributed: one in 10^7 is over REGION_LOST medians.
-constexpr float REGION_WIDE = 1024.0f, REGION_LOST = 24.0f;
+// exponentially distributed: one in 10^7 is over 24 medians (REGION_LOST is
+// wider, a search costs its query as much as 25 others).
+constexpr float REGION_WIDE = 1024.0f, REGION_LOST = 64.0f;
 static_assert(REGION_STACK > 64 + 3 * MAX_LEVELS, "region stack too small");
 
+struct alignas(16) ListedLeaf {
+  float box[6];
+  uint32_t leaf, chunks;  // number, mask of the chunks that may need it
+};
 template <int CHUNKS>
 struct RegionSmem {
-  uint32_t stack[REGION_STACK];
-  float box[6][REGION_LIST];     // listed leaves: box, number, chunks
-  uint32_t leaf[REGION_LIST];
-  uint32_t mask[REGION_LIST];
-  float4 rec[32];                // staged leaf
-  float4 q[32 * CHUNKS];         // queries
-  float d[32 * CHUNKS];          // nearest other point so far (Nearest); d = -1: no query
+  ListedLeaf list[REGION_LIST];
+  alignas(16) float x[32], y[32], z[32];         // staged leaf
+  alignas(16) float qx[32 * CHUNKS], qy[32 * CHUNKS], qz[32 * CHUNKS];  // queries
+  float d[32 * CHUNKS];                          // nearest other point so far (Nearest); d = -1: no query
   int32_t s[32 * CHUNKS], s2[32 * CHUNKS];
-  float cbox[6][CHUNKS];         // chunk boxes
-  float w[CHUNKS];               // largest d of the chunk
+  alignas(16) float chunk[CHUNKS][8];            // box, largest d
+  uint32_t stack[REGION_STACK];
 };
 
 // Nearest other point of a query: (d, s) and s2, the point of the next
@@ -127,6 +132,19 @@ struct Nearest {
   }
 };
 
+// d2_point of four points given as coordinate arrays (paired arithmetic, the
+// same bits); the query twice per register pair.
+__device__ __forceinline__ void d2_point4(const float* x, const float* y, const float* z, unsigned long long qx2,
+                                          unsigned long long qy2, unsigned long long qz2, float (&d)[4]) {
+  const float4 X = *reinterpret_cast<const float4*>(x), Y = *reinterpret_cast<const float4*>(y),
+               Z = *reinterpret_cast<const float4*>(z);
+  const unsigned long long x0 = f2_sub(f2_pack(X.x, X.y), qx2), x1 = f2_sub(f2_pack(X.z, X.w), qx2);
+  const unsigned long long y0 = f2_sub(f2_pack(Y.x, Y.y), qy2), y1 = f2_sub(f2_pack(Y.z, Y.w), qy2);
+  const unsigned long long z0 = f2_sub(f2_pack(Z.x, Z.y), qz2), z1 = f2_sub(f2_pack(Z.z, Z.w), qz2);
+  f2_unpack(f2_fma(z0, z0, f2_fma(x0, x0, f2_mul(y0, y0))), d[0], d[1]);
+  f2_unpack(f2_fma(z1, z1, f2_fma(x1, x1, f2_mul(y1, y1))), d[2], d[3]);
+}
+
 // Queries left to searches of their own (k_radii_hard): sorted positions.
 struct HardList {
   uint32_t* pos;              // room for every point
@@ -149,23 +167,38 @@ __device__ void region_scan(const IndexDev& ix, RegionSmem<CHUNKS>& sm, int64_t 
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   for (int c = 0; c < CHUNKS; ++c) {
-    const float4 q = sm.q[32 * c + lane];
+    const float qx = sm.qx[32 * c + lane], qy = sm.qy[32 * c + lane], qz = sm.qz[32 * c + lane];
+    const unsigned long long qx2 = f2_pack(qx, qx), qy2 = f2_pack(qy, qy), qz2 = f2_pack(qz, qz);
     Nearest N{sm.d[32 * c + lane], sm.s[32 * c + lane], sm.s2[32 * c + lane]};
     const int32_t self = (int32_t)(base + 32 * c + lane);
     for (int e = 0; e < listed; ++e) {
-      if (!((sm.mask[e] >> c) & 1u)) continue;
-      const float m = d2_box(sm.box[0][e], sm.box[1][e], sm.box[2][e], sm.box[3][e], sm.box[4][e], sm.box[5][e],
-                             q.x, q.y, q.z);
+      const float4 lo = *reinterpret_cast<const float4*>(sm.list[e].box);
+      const uint4 hi = *reinterpret_cast<const uint4*>(sm.list[e].box + 4);
+      if (!((hi.w >> c) & 1u)) continue;
+      const float m = d2_box(lo.x, lo.y, lo.z, lo.w, __uint_as_float(hi.x), __uint_as_float(hi.y), qx, qy, qz);
       if (!__ballot_sync(FULL, m <= N.d)) continue;
-      const int64_t start = (int64_t)sm.leaf[e] * ix.leaf;
+      const int64_t start = (int64_t)hi.z * ix.leaf;
       const int cnt = (int)min((int64_t)ix.leaf, ix.n - start);
       __syncwarp();
-      if (lane < cnt) sm.rec[lane] = __ldg(ix.rec + start + lane);
+      const float none = __int_as_float(0x7fffffff);  // NaN, past the leaf's end: within no bound
+      const float4 r = lane < cnt ? __ldg(ix.rec + start + lane) : make_float4(none, none, none, none);
+      sm.x[lane] = r.x;
+      sm.y[lane] = r.y;
+      sm.z[lane] = r.z;
       __syncwarp();
-#pragma unroll 4
-      for (int k = 0; k < cnt; ++k) {
-        const float dd = d2_point(sm.rec[k], q.x, q.y, q.z);
-        if (dd <= N.d) N.consider(dd, (int32_t)start + k, self, ix.perm);
+      for (int k = 0; k < cnt; k += 4) {
+        float d[4];
+        d2_point4(sm.x + k, sm.y + k, sm.z + k, qx2, qy2, qz2, d);
+        if (fminf(fminf(d[0], d[1]), fminf(d[2], d[3])) <= N.d) {
+          // rare: 11 of 170 points are within the bound of any lane
+#pragma unroll 1
+          for (int j = 0; j < 4; ++j) {
+            if (d[0] <= N.d) N.consider(d[0], (int32_t)start + k + j, self, ix.perm);
+            d[0] = d[1];
+            d[1] = d[2];
+            d[2] = d[3];
+          }
+        }
       }
     }
     sm.d[32 * c + lane] = N.d;
@@ -173,7 +206,7 @@ __device__ void region_scan(const IndexDev& ix, RegionSmem<CHUNKS>& sm, int64_t 
     sm.s2[32 * c + lane] = N.s2;
     // distances are >= 0 (or -1 for no query): ordered like signed integers
     const int w = __reduce_max_sync(FULL, __float_as_int(N.d));
-    if (lane == 0) sm.w[c] = __int_as_float(w);
+    if (lane == 0) sm.chunk[c][6] = __int_as_float(w);
   }
   __syncwarp();
 }
@@ -209,24 +242,33 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
       const int64_t s = base + 32 * c + lane;
       const bool active = s < ix.n;
       const float4 q = active ? __ldg(ix.rec + s) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      sm.q[32 * c + lane] = q;
+      const float none = __int_as_float(0x7fffffff);  // a place without a query is near to none
+      sm.qx[32 * c + lane] = active ? q.x : none;
+      sm.qy[32 * c + lane] = active ? q.y : none;
+      sm.qz[32 * c + lane] = active ? q.z : none;
       __syncwarp();
       const int cnt = (int)max((int64_t)0, min((int64_t)32, ix.n - (base + 32 * c)));
+      const unsigned long long qx2 = f2_pack(q.x, q.x), qy2 = f2_pack(q.y, q.y), qz2 = f2_pack(q.z, q.z);
       float d = INF;
       int at = -1;
       bool tie = false;
-#pragma unroll 8
-      for (int k = 0; k < cnt; ++k) {
-        float dd = d2_point(sm.q[32 * c + k], q.x, q.y, q.z);
-        if (k == lane) dd = INF;
-        tie = dd < d ? false : tie || dd == d;
-        at = dd < d ? k : at;
-        d = fminf(d, dd);
+#pragma unroll 2
+      for (int k = 0; k < 32; k += 4) {
+        float dd[4];
+        d2_point4(sm.qx + 32 * c + k, sm.qy + 32 * c + k, sm.qz + 32 * c + k, qx2, qy2, qz2, dd);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (k + j == lane) dd[j] = INF;
+          const bool less = dd[j] < d;
+          tie = !less && (tie || dd[j] == d);
+          at = less ? k + j : at;
+          d = less ? dd[j] : d;
+        }
       }
       Nearest N{d, at >= 0 ? (int32_t)(base + 32 * c) + at : -1, -1};
       if (tie && at >= 0)  // equal nearest distances in the chunk: order them by cloud index
         for (int k = 0; k < cnt; ++k) {
-          const float dd = d2_point(sm.q[32 * c + k], q.x, q.y, q.z);
+          const float dd = d2_point(make_float4(sm.qx[32 * c + k], sm.qy[32 * c + k], sm.qz[32 * c + k], 0.0f), q.x, q.y, q.z);
           if (dd == d) N.consider(dd, (int32_t)(base + 32 * c) + k, (int32_t)s, ix.perm);
         }
       if (active && cnt < 32 && base + 32 * c >= 32)  // a short last chunk: a bound from the chunk before it
@@ -255,16 +297,17 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
       for (int f = 0; f < 6; ++f) {
         const uint32_t o = ordered_bits(here ? lim[f] : f < 3 ? INF : -INF);
         const float v = from_ordered(f < 3 ? __reduce_min_sync(FULL, o) : __reduce_max_sync(FULL, o));
-        if (lane == 0) sm.cbox[f][c] = v;
+        if (lane == 0) sm.chunk[c][f] = v;
       }
       __syncwarp();
-      const float ex = sm.cbox[3][c] - sm.cbox[0][c], ey = sm.cbox[4][c] - sm.cbox[1][c], ez = sm.cbox[5][c] - sm.cbox[2][c];
+      const float* cb = sm.chunk[c];
+      const float ex = cb[3] - cb[0], ey = cb[4] - cb[1], ez = cb[5] - cb[2];
       const float diag2 = ex * ex + ey * ey + ez * ez;
       sm.d[32 * c + lane] = here ? N.d : -1.0f;
       sm.s[32 * c + lane] = N.s;
       sm.s2[32 * c + lane] = N.s2;
       const int w = __reduce_max_sync(FULL, __float_as_int(here ? N.d : -1.0f));
-      if (lane == 0) sm.w[c] = __int_as_float(w);
+      if (lane == 0) sm.chunk[c][6] = __int_as_float(w);
       if (diag2 > REGION_WIDE * __int_as_float(w)) wide |= 1u << c;
     }
     if (lane == 0) sm.stack[0] = 0;
@@ -273,7 +316,7 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
     int sp = 1, listed = 0, scans = 0;
     while (sp > 0) {
       if (listed > REGION_LIST - 32) {
-        if (++scans > REGION_SCANS * (CHUNKS - 1)) {
+        if (++scans > REGION_SCANS<CHUNKS>) {
           // the chunks' bounds are loose as a whole (points strewn over a
           // dense surface of other blocks): a search for every query instead
           for (int c = 0; c < CHUNKS; ++c) {
@@ -297,11 +340,12 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
         for (int f = 0; f < 6; ++f) b[f] = __ldg(g + 4 * f);
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
-          const float gx = fmaxf(fmaxf(__fsub_rn(b[0], sm.cbox[3][c]), __fsub_rn(sm.cbox[0][c], b[3])), 0.0f);
-          const float gy = fmaxf(fmaxf(__fsub_rn(b[1], sm.cbox[4][c]), __fsub_rn(sm.cbox[1][c], b[4])), 0.0f);
-          const float gz = fmaxf(fmaxf(__fsub_rn(b[2], sm.cbox[5][c]), __fsub_rn(sm.cbox[2][c], b[5])), 0.0f);
+          const float4 u = *reinterpret_cast<const float4*>(sm.chunk[c]), v = *reinterpret_cast<const float4*>(sm.chunk[c] + 4);
+          const float gx = fmaxf(fmaxf(__fsub_rn(b[0], u.w), __fsub_rn(u.x, b[3])), 0.0f);
+          const float gy = fmaxf(fmaxf(__fsub_rn(b[1], v.x), __fsub_rn(u.y, b[4])), 0.0f);
+          const float gz = fmaxf(fmaxf(__fsub_rn(b[2], v.y), __fsub_rn(u.z, b[5])), 0.0f);
           const float m = __fmaf_rn(gz, gz, __fmaf_rn(gx, gx, __fmul_rn(gy, gy)));
-          need |= m <= fminf(sm.w[c], FLT_BIG) ? 1u << c : 0u;  // empty boxes, at +inf, never
+          need |= m <= fminf(v.z, FLT_BIG) ? 1u << c : 0u;  // empty boxes, at +inf, never
         }
       }
       for (unsigned todo = __ballot_sync(FULL, need & wide); todo; todo &= todo - 1u) {
@@ -311,8 +355,8 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
         for (int f = 0; f < 6; ++f) o[f] = __shfl_sync(FULL, b[f], src);
         for (unsigned cs = __shfl_sync(FULL, need & wide, src); cs; cs &= cs - 1u) {
           const int c = __ffs(cs) - 1;
-          const float4 q = sm.q[32 * c + lane];
-          const float m = d2_box(o[0], o[1], o[2], o[3], o[4], o[5], q.x, q.y, q.z);
+          const float m = d2_box(o[0], o[1], o[2], o[3], o[4], o[5], sm.qx[32 * c + lane], sm.qy[32 * c + lane],
+                                 sm.qz[32 * c + lane]);
           if (!__ballot_sync(FULL, m <= sm.d[32 * c + lane]) && lane == src) need &= ~(1u << c);
         }
       }
@@ -331,10 +375,9 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
           sm.stack[sp + __popc(inner & lt)] = 4u * G + 1u + ch;
         } else {
           const int e = listed + __popc(leaves & lt);
-#pragma unroll
-          for (int f = 0; f < 6; ++f) sm.box[f][e] = b[f];
-          sm.leaf[e] = leaf;
-          sm.mask[e] = need;
+          *reinterpret_cast<float4*>(sm.list[e].box) = make_float4(b[0], b[1], b[2], b[3]);
+          *reinterpret_cast<uint4*>(sm.list[e].box + 4) =
+              make_uint4(__float_as_uint(b[4]), __float_as_uint(b[5]), leaf, need);
         }
       }
       sp += __popc(inner);
