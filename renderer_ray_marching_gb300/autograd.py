@@ -13,23 +13,29 @@ from __future__ import annotations
 
 import torch
 
+from . import _abi
+
 
 class RenderFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, renderer, views, colours, xyz, radii):
         dev = colours.device
-        rgb_parts, depth_parts, hit_parts = [], [], []
-        for v in views:
-            frame = {"rgbd": torch.empty((v.height, v.width, 4), dtype=torch.float32, device=dev),
-                     "hit": torch.empty((v.height, v.width), dtype=torch.int32, device=dev)}
-            renderer.render_into(v, frame, device=True)
-            rgb_parts.append(frame["rgbd"].reshape(-1, 4)[:, :3])
-            depth_parts.append(frame["rgbd"].reshape(-1, 4)[:, 3])
-            hit_parts.append(frame["hit"].reshape(-1))
+        if len(views) == 0:
+            raise RuntimeError("no views to render")
+        # all views in one launch, into one buffer (a view after the other)
+        pixels = sum(v.pixels for v in views)
+        rgbd = torch.empty((pixels, 4), dtype=torch.float32, device=dev)
+        hit = torch.empty(pixels, dtype=torch.int32, device=dev)
+        frames = (_abi.RmFrame * len(views))()
+        lo = 0
+        for frame, v in zip(frames, views):
+            frame.rgbd = rgbd.data_ptr() + 16 * lo
+            frame.hit = hit.data_ptr() + 4 * lo
+            lo += v.pixels
+        renderer.render_batch_into(views, frames, device=True)
         renderer.synchronize()
-        rgb = torch.cat(rgb_parts).contiguous()
-        depth = torch.cat(depth_parts).contiguous()
-        hit = torch.cat(hit_parts).contiguous()
+        rgb = rgbd[:, :3].contiguous()
+        depth = rgbd[:, 3].contiguous()
         ctx.renderer = renderer
         ctx.views = views
         ctx.n = xyz.shape[0]

@@ -208,7 +208,7 @@ void rm_ctx_destroy(rm_ctx* ctx) {
   c.drop_graph();
   DevBuf* bufs[] = {&c.pos, &c.radii_clamped, &c.rec, &c.col, &c.perm, &c.groups,
                     &c.keys, &c.vals, &c.sort_counts,
-                    &c.scan_sums, &c.scratch_bounds, &c.bucket_i, &c.scalars, &c.staging_in, &c.staging_out,
+                    &c.scan_sums, &c.bucket_i, &c.scalars, &c.staging_in, &c.staging_out,
                     &c.views, &c.frame_bufs, &c.queue, &c.tail};
   for (DevBuf* b : bufs) b->release();
   if (c.pinned_views) cudaFreeHost(c.pinned_views);
@@ -265,8 +265,7 @@ rm_status rm_index_build(rm_ctx* ctx) {
       c.depth = 0;
       return RM_OK;
     }
-    if (!build_index(c)) return RM_ERR_INVALID;
-    CK(cudaStreamSynchronize(c.stream));
+    if (!build_index(c)) return RM_ERR_INVALID;  // synchronises
     return RM_OK;
   });
 }
@@ -330,7 +329,8 @@ rm_status rm_radii_compute(rm_ctx* ctx, float max_radius, float* radii_out, int3
       dn = nn_out ? reinterpret_cast<int32_t*>(c.staging_out.ptr<float>() + n) : nullptr;
     }
     reserve_tail(c);
-    CK(cudaMemsetAsync(err_counter(c), 0, 8, c.stream));
+    // largest radius, search counters and errors
+    CK(cudaMemsetAsync(c.scalars.ptr<unsigned long long>() + 4, 0, 5 * 8, c.stream));
     launch_radii(c, max_radius, dr, dn);  // also sets the records' radii
     CK(cudaGetLastError());
     // the largest radius and the error counts in one read

@@ -48,6 +48,14 @@ __host__ __device__ __forceinline__ int64_t group_offset(int lvl) {
   return (int64_t)(((1u << (2 * lvl)) - 1u) / 3u);
 }
 
+// Floats as unsigned integers of the same order, and back.
+__device__ __forceinline__ uint32_t ordered_bits(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
+}
+__host__ __device__ __forceinline__ uint32_t from_ordered_bits(uint32_t o) { return o & 0x80000000u ? o ^ 0x80000000u : ~o; }
+__device__ __forceinline__ float from_ordered(uint32_t o) { return __uint_as_float(from_ordered_bits(o)); }
+
 __device__ __forceinline__ float d2_point(float4 c, float qx, float qy, float qz) {
   float dx = __fsub_rn(c.x, qx);
   float dy = __fsub_rn(c.y, qy);
@@ -681,9 +689,8 @@ struct PacketQueue {
 // (broadcast loads) while every lane updates its own list.  All 32 lanes
 // call it with warp-uniform control flow; inactive lanes only follow along.
 // Returns false if the node budget was hit (cannot happen with an exact
-// bound).  Nodes are addressed by their group's level-order index G: the
-// children of G have groups 4G + 1 + c, and a stack entry holds
-// (level << 28) | G, so no level offset is computed on the walk.
+// bound).  Nodes are addressed by their group's level-order index G (the
+// children of G have groups 4G + 1 + c), which also tells the last level.
 //
 // The walk is best-first.  A depth-first walk finishes the leading lane's
 // subtree before anything else, so lanes whose nearest points lie in another
@@ -762,7 +769,6 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
       qcode = code;
     }
   };
-  int lvl = 0;
   uint32_t G = 0;
   const unsigned nodes0 = nodes;
   while (true) {
@@ -782,23 +788,21 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
     unsigned mine = 0;
     if (active) mine = (m0 <= w ? 1u : 0u) | (m1 <= w ? 2u : 0u) | (m2 <= w ? 4u : 0u) | (m3 <= w ? 8u : 0u);
     const unsigned needm = __reduce_or_sync(FULL, mine);
-    if (needm != 0 && lvl + 1 != ix.depth && !dfs) {
+    if (needm != 0 && G < last_first && !dfs) {
       // Inner node, best-first.  Keys are the leading lane's box distances:
       // the walk descends into the nearest needed child unless a queued node
       // is nearer still, and queues the other needed children (the queue
       // keeps them in key order, so no ordering network is needed here).
       const uint32_t child0 = 4u * G + 1u;
-      const uint32_t lcode = (uint32_t)(lvl + 1) << 28;
       if (!(needm & (needm - 1u))) {
         // one child (about 35% of expansions): one shuffle
         const int c = __ffs(needm) - 1;
         const float kc = __shfl_sync(FULL, c == 0 ? m0 : c == 1 ? m1 : c == 2 ? m2 : m3, leader);
         if (qn == 0 || kc <= __shfl_sync(FULL, qkey, 0)) {
-          lvl = lvl + 1;
           G = child0 + (uint32_t)c;
           continue;
         }
-        qpush(kc, lcode | (child0 + (uint32_t)c));
+        qpush(kc, child0 + (uint32_t)c);
       } else {
         const float k0 = __shfl_sync(FULL, m0, leader), k1 = __shfl_sync(FULL, m1, leader);
         const float k2 = __shfl_sync(FULL, m2, leader), k3 = __shfl_sync(FULL, m3, leader);
@@ -809,14 +813,13 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
         const int cf = k23 < k01 ? c23 : c01;  // nearest needed child, ties to the lower index
         const bool down = qn == 0 || fminf(k01, k23) <= __shfl_sync(FULL, qkey, 0);
         const unsigned topush = down ? (needm & ~(1u << cf)) : needm;
-        if (topush & 1u) qpush(k0, lcode | child0);
-        if (topush & 2u) qpush(k1, lcode | (child0 + 1u));
-        if (topush & 4u) qpush(k2, lcode | (child0 + 2u));
-        if (topush & 8u) qpush(k3, lcode | (child0 + 3u));
+        if (topush & 1u) qpush(k0, child0);
+        if (topush & 2u) qpush(k1, child0 + 1u);
+        if (topush & 4u) qpush(k2, child0 + 2u);
+        if (topush & 8u) qpush(k3, child0 + 3u);
         if (down) {
           if (sp + fsp > PSTACK) return false;
           __syncwarp();
-          lvl = lvl + 1;
           G = child0 + (uint32_t)cf;
           continue;
         }
@@ -838,7 +841,7 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
         order = __shfl_sync(FULL, (unsigned)o0 | ((unsigned)o1 << 2) | ((unsigned)o2 << 4) | ((unsigned)o3 << 6),
                             leader);
       }
-      if (lvl + 1 == ix.depth) {
+      if (G >= last_first) {
         const uint32_t lbase = (G - last_first) * 4u;
 #pragma unroll 1  // one copy of the scan: four cost more in instruction fetch
         for (int t = 0; t < 4; ++t) {
@@ -866,6 +869,7 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
           }
           __syncwarp();
           if (active) {
+#pragma unroll 1
             for (int k = 0; k < cnt; k += 4) {
               float d0, d1, d2, d3;
               {
@@ -893,18 +897,16 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
         const int tf = __ffs(om) - 1;
         const unsigned rest = om & (om - 1u);
         const uint32_t child0 = 4u * G + 1u;
-        const uint32_t lcode = (uint32_t)(lvl + 1) << 28;
-        if (dfs) {
+          if (dfs) {
           // depth-first: descend into the nearest needed child; lanes 0-3
           // push the others, farthest deepest so the nearest pops first
           if (sp + fsp + 3 > PSTACK) return false;
           if (lane < 4 && ((rest >> lane) & 1u)) {
             const int slot = sp + __popc(rest >> (lane + 1));
-            ps.code[slot] = lcode | (child0 + ((order >> (2 * lane)) & 3u));
+            ps.code[slot] = child0 + ((order >> (2 * lane)) & 3u);
           }
           sp += __popc(rest);
           __syncwarp();
-          lvl = lvl + 1;
           G = child0 + ((order >> (2 * tf)) & 3u);
           continue;
         }
@@ -931,7 +933,7 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
         // queue entry (87% still needed when taken), such a node is worth
         // re-testing before its expansion: its box is lane (G - 1) & 3 of
         // its parent's group (about 14 fewer expansions per warp step, +1%).
-        const uint32_t pG = code & 0x0fffffffu;
+        const uint32_t pG = code;
         const float* pg = reinterpret_cast<const float*>(ix.groups + (size_t)GROUP_F4 * ((pG - 1u) >> 2));
         const int c = (int)((pG - 1u) & 3u);
         float md = INF;
@@ -949,8 +951,7 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
       // children against the current bounds, and a child's box lies inside
       // its parent's, so a node that is no longer needed yields no needed
       // child (one dependent load fewer per taken node, measured +1.2%)
-      lvl = (int)(code >> 28);
-      G = code & 0x0fffffffu;
+      G = code;
       found = true;
       break;
     }

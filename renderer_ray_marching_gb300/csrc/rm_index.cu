@@ -3,7 +3,7 @@
 // x, y and z separately and syncs with the host once per tree level).
 //
 // Build, all on the device with no host round trip between passes:
-//   1. bounds:   block-reduced min/max of the cloud (+ a non-finite flag);
+//   1. bounds:   of the cloud, kept when it was packed (+ a non-finite flag);
 //   2. keys:     32-bit Hilbert-curve key of each point's cubic cell;
 //   3. sort:     LSD radix sort of (key, cloud index), 4 passes of 8 bits,
 //                stable warp-level ranking by digit votes;
@@ -26,83 +26,52 @@
 
 namespace rm {
 
-// ---------------------------------------------------------------- bounds
-// Points as float4: x, y, z and the packed colour in .w.
-__global__ void k_pack(const float* __restrict__ xyz, int stride, const uint8_t* __restrict__ rgb, int64_t n,
-                       float4* __restrict__ pos) {
+// ---------------------------------------------------------------- points
+// Points as float4: x, y, z and the packed colour in .w; and the cloud's
+// bounds on the way: bounds[0..2] lower and [3..5] upper corner as
+// ordered_bits (set to the ends of the range before), [6] nonzero if a
+// coordinate is not finite.
+constexpr int PACK_THREADS = 256;
+__global__ void __launch_bounds__(PACK_THREADS)
+k_pack(const float* __restrict__ xyz, int stride, const uint8_t* __restrict__ rgb, int64_t n,
+       float4* __restrict__ pos, uint32_t* __restrict__ bounds) {
+  float lo[3] = {INFINITY, INFINITY, INFINITY};
+  float hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const float* p = xyz + i * stride;
-    uint32_t c = 0xffffffu;
-    if (rgb) c = (uint32_t)rgb[3 * i] | ((uint32_t)rgb[3 * i + 1] << 8) | ((uint32_t)rgb[3 * i + 2] << 16);
-    pos[i] = make_float4(p[0], p[1], p[2], __uint_as_float(c));
-  }
-}
-
-// Per-block partial bounds: out[block * 8 + {0..5}] = lo xyz, hi xyz;
-// [6] = 1 if a non-finite coordinate was seen.
-__global__ void k_bounds_partial(const float4* __restrict__ pos, int64_t n,
-                                 float* __restrict__ out) {
-  float lo[3] = {INFINITY, INFINITY, INFINITY};
-  float hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  float bad = 0.0f;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float4 p = pos[i];
-    float c[3] = {p.x, p.y, p.z};
+    const float c[3] = {p[0], p[1], p[2]};
+    uint32_t u = 0xffffffu;
+    if (rgb) u = (uint32_t)rgb[3 * i] | ((uint32_t)rgb[3 * i + 1] << 8) | ((uint32_t)rgb[3 * i + 2] << 16);
+    pos[i] = make_float4(c[0], c[1], c[2], __uint_as_float(u));
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      if (!isfinite(c[a])) bad = 1.0f;
+      bad |= !isfinite(c[a]);
       lo[a] = fminf(lo[a], c[a]);
       hi[a] = fmaxf(hi[a], c[a]);
     }
   }
-  __shared__ float sh[7][32];
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ uint32_t sh[6][PACK_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], off));
-      hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], off));
+  for (int a = 0; a < 3; ++a) {
+    const uint32_t l = __reduce_min_sync(0xffffffffu, ordered_bits(lo[a]));
+    const uint32_t h = __reduce_max_sync(0xffffffffu, ordered_bits(hi[a]));
+    if (lane == 0) {
+      sh[a][warp] = l;
+      sh[3 + a][warp] = h;
     }
-    bad = fmaxf(bad, __shfl_xor_sync(0xffffffffu, bad, off));
   }
-  if (lane == 0) {
-    for (int a = 0; a < 3; ++a) {
-      sh[a][warp] = lo[a];
-      sh[3 + a][warp] = hi[a];
-    }
-    sh[6][warp] = bad;
+  const int any_bad = __syncthreads_or(bad);
+  if (threadIdx.x < 6) {
+    uint32_t v = sh[threadIdx.x][0];
+    for (int w = 1; w < PACK_THREADS / 32; ++w)
+      v = threadIdx.x < 3 ? min(v, sh[threadIdx.x][w]) : max(v, sh[threadIdx.x][w]);
+    if (threadIdx.x < 3) atomicMin(bounds + threadIdx.x, v);
+    else atomicMax(bounds + threadIdx.x, v);
   }
-  __syncthreads();
-  if (threadIdx.x < 7) {
-    int nw = blockDim.x >> 5;
-    float v = sh[threadIdx.x][0];
-    for (int w = 1; w < nw; ++w) {
-      float x = sh[threadIdx.x][w];
-      v = (threadIdx.x < 3) ? fminf(v, x) : fmaxf(v, x);
-    }
-    out[blockIdx.x * 8 + threadIdx.x] = v;
-  }
-}
-
-// Warp a reduces component a of the partials.
-__global__ void k_bounds_final(const float* __restrict__ part, int nblocks,
-                               float* __restrict__ out) {
-  const int a = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (a >= 7) return;
-  float v = part[a];
-  for (int b = lane; b < nblocks; b += 32) {
-    const float x = part[b * 8 + a];
-    v = (a < 3) ? fminf(v, x) : fmaxf(v, x);
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    const float x = __shfl_xor_sync(0xffffffffu, v, off);
-    v = (a < 3) ? fminf(v, x) : fmaxf(v, x);
-  }
-  if (lane == 0) out[a] = v;
+  if (any_bad && threadIdx.x == 0) atomicOr(bounds + 6, 1u);
 }
 
 // ---------------------------------------------------------------- curve keys
@@ -154,12 +123,12 @@ __device__ __forceinline__ uint32_t curve_key(uint32_t x, uint32_t y, uint32_t z
 // the bounds.
 struct CurveGrid {
   float lo[3], sc;
-  __device__ __forceinline__ explicit CurveGrid(const float* __restrict__ bounds) {
+  __device__ __forceinline__ explicit CurveGrid(const uint32_t* __restrict__ bounds) {
     float side = 1e-30f;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-      lo[a] = bounds[a];
-      side = fmaxf(side, bounds[3 + a] - bounds[a]);
+      lo[a] = from_ordered(bounds[a]);
+      side = fmaxf(side, from_ordered(bounds[3 + a]) - lo[a]);
     }
     sc = (float)((1 << CURVE_BITS) - 1) / side;
   }
@@ -173,7 +142,7 @@ struct CurveGrid {
 
 // Points per coarse cell (2^g along a side), for the keys below: of every 256
 // points 32 are counted.
-__global__ void k_coarse_count(const float4* __restrict__ pos, int64_t n, const float* __restrict__ bounds, int g,
+__global__ void k_coarse_count(const float4* __restrict__ pos, int64_t n, const uint32_t* __restrict__ bounds, int g,
                                uint32_t* __restrict__ count) {
   const CurveGrid grid(bounds);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;; t += (int64_t)gridDim.x * blockDim.x) {
@@ -192,7 +161,7 @@ __global__ void k_coarse_count(const float4* __restrict__ pos, int64_t n, const 
 // nearby has to look into.  A point whose coarse cell holds under an eighth
 // of the points of the cell beyond a near face (at most a quarter cell away)
 // takes its key from that cell's edge.
-__global__ void k_curve_keys(const float4* __restrict__ pos, int64_t n, const float* __restrict__ bounds, int g,
+__global__ void k_curve_keys(const float4* __restrict__ pos, int64_t n, const uint32_t* __restrict__ bounds, int g,
                              const uint32_t* __restrict__ count, uint32_t* __restrict__ keys) {
   const CurveGrid grid(bounds);
   const int sh = CURVE_BITS - g;
@@ -242,6 +211,9 @@ constexpr int SORT_ITEMS = 16;
 constexpr int SORT_TILE = SORT_THREADS * SORT_ITEMS;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
 constexpr int RADIX = 256;
+// Up to this many tiles the scatter sums the counts itself: 2 launches a pass
+// instead of 5, 66 -> 43 us for the whole sort at 100k points.
+constexpr int64_t SORT_OWN_SCAN = 64;
 
 __global__ void __launch_bounds__(SORT_THREADS)
 k_sort_hist(const uint32_t* __restrict__ keys, int64_t n, int shift, int64_t ntiles,
@@ -349,8 +321,7 @@ k_scan_add(uint32_t* __restrict__ data, int64_t len, const uint32_t* __restrict_
   }
 }
 
-// Exclusive prefix over RADIX digit counts held by the first RADIX threads;
-// all threads of the block call it.
+// Exclusive prefix over RADIX digit counts, one per thread.
 __device__ __forceinline__ uint32_t digit_prefix(uint32_t v, uint32_t* warp_sums) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t x = v;
@@ -359,10 +330,10 @@ __device__ __forceinline__ uint32_t digit_prefix(uint32_t v, uint32_t* warp_sums
     const uint32_t y = __shfl_up_sync(0xffffffffu, x, off);
     if (lane >= off) x += y;
   }
-  if (lane == 31 && warp < RADIX / 32) warp_sums[warp] = x;
+  if (lane == 31) warp_sums[warp] = x;
   __syncthreads();
   uint32_t before = 0;
-  for (int w = 0; w < warp && w < RADIX / 32; ++w) before += warp_sums[w];
+  for (int w = 0; w < warp; ++w) before += warp_sums[w];
   return before + x - v;
 }
 
@@ -373,7 +344,9 @@ struct SortSmem {
   uint32_t key[SORT_TILE], val[SORT_TILE];
 };
 
-template <bool FIRST>
+// FIRST: the values are the positions.  SCANNED: `offsets` holds the scanned
+// counts; else the counts themselves, and every CTA sums what precedes it.
+template <bool FIRST, bool SCANNED>
 __global__ void __launch_bounds__(SORT_THREADS, 4)
 k_sort_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                int64_t n, int shift, int64_t ntiles, const uint32_t* __restrict__ offsets,
@@ -413,14 +386,27 @@ k_sort_scatter(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict_
   }
   __syncthreads();
   // places within the tile: digits in order, and within a digit the warps
+  static_assert(SORT_THREADS == RADIX, "one digit per thread");
   uint32_t total = 0;
   const int d = threadIdx.x;
-  if (d < RADIX)
 #pragma unroll
-    for (int w = 0; w < SORT_WARPS; ++w) total += sm.cnt[w][d];
-  const uint32_t first = digit_prefix(d < RADIX ? total : 0u, sm.sums);
-  if (d < RADIX) {
-    sm.base[d] = offsets[(int64_t)d * ntiles + blockIdx.x] - first;
+  for (int w = 0; w < SORT_WARPS; ++w) total += sm.cnt[w][d];
+  const uint32_t first = digit_prefix(total, sm.sums);
+  uint32_t place = 0;
+  if (!SCANNED) {
+    uint32_t mine = 0, all = 0;
+    for (int64_t t = 0; t < ntiles; ++t) {
+      const uint32_t v = __ldg(offsets + (int64_t)d * ntiles + t);
+      all += v;
+      mine += t < (int64_t)blockIdx.x ? v : 0u;
+    }
+    __syncthreads();  // sums are read again
+    place = digit_prefix(all, sm.sums) + mine;
+  } else {
+    place = offsets[(int64_t)d * ntiles + blockIdx.x];
+  }
+  {
+    sm.base[d] = place - first;
     uint32_t run = first;
 #pragma unroll
     for (int w = 0; w < SORT_WARPS; ++w) {
@@ -778,7 +764,10 @@ static int grid_for(int64_t n, int threads, int max_blocks = 152 * 32) {
 }
 
 void launch_pack(Ctx& c, const float* xyz, int stride, const uint8_t* rgb, int64_t n) {
-  k_pack<<<grid_for(n, 256), 256, 0, c.stream>>>(xyz, stride, rgb, n, c.pos.ptr<float4>());
+  uint32_t* bounds = c.scalars.ptr<uint32_t>();
+  CK(cudaMemsetAsync(bounds, 0xff, 3 * 4, c.stream));
+  CK(cudaMemsetAsync(bounds + 3, 0, 4 * 4, c.stream));
+  k_pack<<<grid_for(n, PACK_THREADS), PACK_THREADS, 0, c.stream>>>(xyz, stride, rgb, n, c.pos.ptr<float4>(), bounds);
 }
 
 void launch_clamp_radii_only(Ctx& c, const float* in, float max_radius) {
@@ -822,20 +811,7 @@ void refresh_max_radius(Ctx& c) {
 bool build_index(Ctx& c) {
   const int64_t n = c.n;
   cudaStream_t st = c.stream;
-  // bounds
-  int nb = grid_for(n, 256, 1024);
-  c.scratch_bounds.reserve((size_t)nb * 8 * sizeof(float));
-  k_bounds_partial<<<nb, 256, 0, st>>>(c.pos.ptr<float4>(), n, c.scratch_bounds.ptr<float>());
-  k_bounds_final<<<1, 7 * 32, 0, st>>>(c.scratch_bounds.ptr<float>(), nb, c.scalars.ptr<float>());
-  float hb[8];
-  CK(cudaMemcpyAsync(hb, c.scalars.ptr<float>(), 8 * sizeof(float), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  if (hb[6] != 0.0f) {
-    c.err = "cloud contains non-finite coordinates";
-    return false;
-  }
-  for (int a = 0; a < 6; ++a) c.bounds[a] = hb[a];
-
+  uint32_t* bounds = c.scalars.ptr<uint32_t>();
   // keys
   // Coarse cells of about 500 points where points lie on surfaces (about
   // 2.5 cells across occupied per cell of a face), half a block of the tree.
@@ -846,30 +822,38 @@ bool build_index(Ctx& c) {
   c.vals.reserve((size_t)c.half * 8);
   uint32_t* coarse = c.key(1);  // counted in the sort's second buffer
   CK(cudaMemsetAsync(coarse, 0, (size_t)4 << (3 * g), st));
-  k_coarse_count<<<grid_for((n + 7) / 8, 256), 256, 0, st>>>(c.pos.ptr<float4>(), n, c.scalars.ptr<float>(), g, coarse);
-  k_curve_keys<<<grid_for(n, 256), 256, 0, st>>>(c.pos.ptr<float4>(), n, c.scalars.ptr<float>(), g, coarse,
+  k_coarse_count<<<grid_for((n + 7) / 8, 256), 256, 0, st>>>(c.pos.ptr<float4>(), n, bounds, g, coarse);
+  k_curve_keys<<<grid_for(n, 256), 256, 0, st>>>(c.pos.ptr<float4>(), n, bounds, g, coarse,
                                                  c.key(0));
   // radix sort, 32-bit keys: shifts 0, 8, 16, 24
   int64_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
   int64_t clen = ntiles * RADIX;
   int64_t nscan = (clen + SCAN_TILE - 1) / SCAN_TILE;
   c.sort_counts.reserve((size_t)clen * 4);
-  c.scan_sums.reserve((size_t)(nscan + 1) * 4);
+  c.scan_sums.reserve((size_t)(nscan + 1) * 4 + 1024);  // also the buckets' cursors (rm_radii.cu)
   int cur = 0;
   for (int shift = 0; shift < 32; shift += 8) {
     uint32_t* cnt = c.sort_counts.ptr<uint32_t>();
     k_sort_hist<<<(unsigned)ntiles, SORT_THREADS, 0, st>>>(c.key(cur), n, shift, ntiles, cnt);
-    k_scan_tiles<<<(unsigned)nscan, SCAN_THREADS, 0, st>>>(cnt, clen, c.scan_sums.ptr<uint32_t>());
-    k_scan_sums<<<1, SCAN_THREADS, 0, st>>>(c.scan_sums.ptr<uint32_t>(), nscan);
-    k_scan_add<<<(unsigned)nscan, SCAN_THREADS, 0, st>>>(cnt, clen, c.scan_sums.ptr<uint32_t>());
+    const bool scanned = ntiles > SORT_OWN_SCAN;
+    if (scanned) {
+      k_scan_tiles<<<(unsigned)nscan, SCAN_THREADS, 0, st>>>(cnt, clen, c.scan_sums.ptr<uint32_t>());
+      k_scan_sums<<<1, SCAN_THREADS, 0, st>>>(c.scan_sums.ptr<uint32_t>(), nscan);
+      k_scan_add<<<(unsigned)nscan, SCAN_THREADS, 0, st>>>(cnt, clen, c.scan_sums.ptr<uint32_t>());
+    }
     auto scatter = [&](auto kern) {
       CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SortSmem)));
       kern<<<(unsigned)ntiles, SORT_THREADS, sizeof(SortSmem), st>>>(
           c.key(cur), c.val(cur), n, shift, ntiles, cnt,
           c.key(cur ^ 1), c.val(cur ^ 1));
     };
-    if (shift == 0) scatter(k_sort_scatter<true>);
-    else scatter(k_sort_scatter<false>);
+    if (scanned) {
+      if (shift == 0) scatter(k_sort_scatter<true, true>);
+      else scatter(k_sort_scatter<false, true>);
+    } else {
+      if (shift == 0) scatter(k_sort_scatter<true, false>);
+      else scatter(k_sort_scatter<false, false>);
+    }
     cur ^= 1;
   }
   // leaves and tree
@@ -908,7 +892,21 @@ bool build_index(Ctx& c) {
   c.depth = depth;
   c.nleaves = nleaves;
   CK(cudaGetLastError());
-  if (c.have_radii) refresh_max_radius(c);
+  if (c.have_radii) launch_max_radius(c);
+  // bounds, the non-finite flag and the largest radius in one read (an index
+  // over non-finite points is built but not used)
+  uint32_t hb[9];
+  CK(cudaMemcpyAsync(hb, bounds, sizeof(hb), cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  if (hb[6] != 0) {
+    c.err = "cloud contains non-finite coordinates";
+    return false;
+  }
+  for (int a = 0; a < 6; ++a) {
+    const uint32_t u = from_ordered_bits(hb[a]);
+    memcpy(&c.bounds[a], &u, sizeof(u));
+  }
+  if (c.have_radii) set_max_radius(c, hb[8]);
   c.have_index = true;
   return true;
 }

@@ -101,9 +101,10 @@ struct Ctx {
   int64_t half = 0;
   uint32_t* key(int i) const { return keys.ptr<uint32_t>() + i * half; }
   uint32_t* val(int i) const { return vals.ptr<uint32_t>() + i * half; }
-  DevBuf sort_counts, scan_sums, scratch_bounds;
+  DevBuf sort_counts, scan_sums;
   DevBuf bucket_i;       // cloud indices of radii on their way to cloud order
-  DevBuf scalars;        // [0..6] bounds + flag, [8] max radius bits, [16..] counters
+  DevBuf scalars;        // words 0-6 bounds + flag; 64-bit [4] largest radius bits, [5, 6] radii search,
+                         // [8] its errors, [16..] counters
   DevBuf staging_in, staging_out;
   DevBuf views;          // ViewDev table
   DevBuf frame_bufs;     // device outputs for host-side frames

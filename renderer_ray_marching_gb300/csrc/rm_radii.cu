@@ -211,14 +211,6 @@ __device__ void region_scan(const IndexDev& ix, RegionSmem<CHUNKS>& sm, int64_t 
   __syncwarp();
 }
 
-__device__ __forceinline__ uint32_t ordered_bits(float f) {
-  const uint32_t u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : u | 0x80000000u;
-}
-__device__ __forceinline__ float from_ordered(uint32_t u) {
-  return __uint_as_float((u & 0x80000000u) ? u & 0x7fffffffu : ~u);
-}
-
 template <int CHUNKS>
 __global__ void __launch_bounds__(32 * RADII_WARPS)
 k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ nn_sorted,
@@ -607,11 +599,11 @@ void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
     // free once the index is built)
     float* r_sorted = reinterpret_cast<float*>(c.key(0));
     int32_t* nn_sorted = reinterpret_cast<int32_t*>(c.key(1));
-    unsigned long long* next = c.queue.ptr<unsigned long long>() + 1;
-    // [1] region counter, [2] handed-over queries (positions in the sort's
-    // value buffer, free like its key buffers)
+    // scalars, cleared by the caller: [4] largest radius, [5] region counter,
+    // [6] handed-over queries (positions in the sort's value buffer, free like
+    // its key buffers)
+    unsigned long long* next = c.scalars.ptr<unsigned long long>() + 5;
     const HardList hard{c.val(0), next + 1};
-    CK(cudaMemsetAsync(next, 0, 2 * sizeof(unsigned long long), c.stream));
     auto go = [&](auto kern, int chunks) {
       int per_sm = 0;
       CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * RADII_WARPS, 0));
@@ -632,7 +624,7 @@ void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
     } else {
       int shift = 0;
       while ((c.n - 1) >> shift >= BUCKETS) ++shift;
-      uint32_t* cursor = c.scratch_bounds.ptr<uint32_t>();
+      uint32_t* cursor = c.scan_sums.ptr<uint32_t>();
       CK(cudaMemsetAsync(cursor, 0, BUCKETS * 4, c.stream));
       c.bucket_i.reserve((size_t)c.n * 4);
       int32_t* to_i = c.bucket_i.ptr<int32_t>();
@@ -645,7 +637,6 @@ void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
       k_from_buckets<<<tiles, BUCKET_THREADS, 0, c.stream>>>(to_i, apart, c.n, pairs);
     }
     unsigned* largest = c.scalars.ptr<unsigned>() + 8;
-    CK(cudaMemsetAsync(largest, 0, sizeof(unsigned), c.stream));
     k_split<<<std::min(blocks_for(c, c.n, 256), c.sm_count * 8), 256, 0, c.stream>>>(pairs, c.n, max_radius, radii_out, nn_out,
                                                            c.radii_clamped.ptr<float>(), largest);
   } else {

@@ -35,9 +35,7 @@ class View:
 
     def to_c(self) -> _abi.RmView:
         v = _abi.RmView()
-        m = np.ascontiguousarray(self.cam2world, np.float32).reshape(16)
-        for i in range(16):
-            v.cam2world[i] = float(m[i])
+        v.cam2world[:] = np.asarray(self.cam2world, np.float32).reshape(16).tolist()
         v.width = int(self.width)
         v.height = int(self.height)
         v.fov = float(np.float32(self.fov))
