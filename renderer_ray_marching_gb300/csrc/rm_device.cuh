@@ -458,30 +458,35 @@ __device__ bool knn_search(const IndexDev& ix, float qx, float qy, float qz, Lis
 //
 // The warp's list: lane j holds the j-th nearest point as a 64-bit key
 // (bits of d2, cloud index), so keys order exactly like (d2, cloud index),
-// and its sorted position s.  Unfilled entries have s = -1 and a key above
-// every point's.
+// and with POS its sorted position s.  Unfilled entries have the cloud index
+// 2^32 - 1 (s = -1), above every point's at the same distance.
+template <bool POS>
 struct WarpList {
   unsigned long long key;
   int32_t s;
   __device__ __forceinline__ float dist(int j) const {
     return __uint_as_float(__shfl_sync(0xffffffffu, (unsigned)(key >> 32), j));
   }
+  // this lane's cloud index, -1: unfilled
+  __device__ __forceinline__ int32_t index() const { return (int32_t)(unsigned)key; }
   // empty list whose entries stand at distance `bound`
   __device__ __forceinline__ void clear(float bound) {
     key = ((unsigned long long)__float_as_uint(bound) << 32) | 0xffffffffu;
     s = -1;
   }
-  __device__ __forceinline__ void exchange(unsigned long long& k, int32_t& v, int j, bool keep_min) const {
+  static __device__ __forceinline__ void exchange(unsigned long long& k, int32_t& v, int j, bool keep_min) {
     const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, j);
-    const int32_t ov = __shfl_xor_sync(0xffffffffu, v, j);
-    if ((ok < k) == keep_min) {
-      k = ok;
-      v = ov;
+    const bool take = (ok < k) == keep_min;
+    if (POS) {
+      const int32_t ov = __shfl_xor_sync(0xffffffffu, v, j);
+      v = take ? ov : v;
     }
+    k = take ? ok : k;
   }
   // Takes one candidate per lane (d2, sorted position) where `take` is set.
   // A few go in one by one; many are sorted by a bitonic network and merged
-  // with the list (26 exchange steps, the price of about ten insertions).
+  // with the list (26 exchange steps, the price of about ten insertions;
+  // the first ones need no merge).
   __device__ __forceinline__ void offer(bool take, float d2, int32_t pos, const int32_t* __restrict__ perm) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -493,29 +498,36 @@ struct WarpList {
       for (; todo; todo &= todo - 1u) {
         const int src = __ffs(todo) - 1;
         const unsigned long long ck = __shfl_sync(FULL, k, src);
-        const int32_t cs = __shfl_sync(FULL, pos, src);
-        const bool below = key < ck;
+        const int at = __popc(__ballot_sync(FULL, key < ck));
         const unsigned long long uk = __shfl_up_sync(FULL, key, 1);
-        const int32_t us = __shfl_up_sync(FULL, s, 1);
-        const int at = __popc(__ballot_sync(FULL, below));
-        if (lane >= at) {
-          key = lane == at ? ck : uk;
-          s = lane == at ? cs : us;
+        if (POS) {
+          const int32_t cs = __shfl_sync(FULL, pos, src), us = __shfl_up_sync(FULL, s, 1);
+          if (lane >= at) s = lane == at ? cs : us;
         }
+        if (lane >= at) key = lane == at ? ck : uk;
       }
       return;
     }
+    if (POS) pos = take ? pos : -1;
 #pragma unroll
     for (int size = 2; size <= 32; size *= 2)
 #pragma unroll
       for (int j = size / 2; j > 0; j /= 2) exchange(k, pos, j, ((lane & j) == 0) == ((lane & size) == 0));
+    if (__ballot_sync(FULL, index() != -1) == 0) {
+      if (k < key) {  // an empty list: the sorted candidates, up to its bound
+        key = k;
+        if (POS) s = pos;
+      }
+      return;
+    }
     // the 32 smallest of both, as a bitonic sequence
     const unsigned long long rk = __shfl_xor_sync(FULL, k, 31);
-    const int32_t rs = __shfl_xor_sync(FULL, pos, 31);
-    if (rk < key) {
-      key = rk;
-      s = rs;
+    const bool less = rk < key;
+    if (POS) {
+      const int32_t rs = __shfl_xor_sync(FULL, pos, 31);
+      s = less ? rs : s;
     }
+    key = less ? rk : key;
 #pragma unroll
     for (int j = 16; j > 0; j /= 2) exchange(key, s, j, (lane & j) == 0);
   }
@@ -543,7 +555,8 @@ struct WarpPool {
 // 16 grandchildren are 512 consecutive bytes, and 32 lanes test the
 // grandchildren of two nodes at once (an odd depth takes its first step
 // alone).  Then the leaves among them are measured, 32 points at a time.
-__device__ __forceinline__ void warp_knn(const IndexDev& ix, float qx, float qy, float qz, int k, WarpList& L,
+template <bool POS>
+__device__ __forceinline__ void warp_knn(const IndexDev& ix, float qx, float qy, float qz, int k, WarpList<POS>& L,
                                          WarpPool& pool) {
   const unsigned FULL = 0xffffffffu;
   const float INF = __int_as_float(0x7f800000);

@@ -202,7 +202,7 @@ __device__ __forceinline__ void march_one(const IndexDev& ix, const ClipBox& cli
     if (lane < KNN && seed >= 0) d = d2_point(__ldg(ix.rec + seed), px, py, pz);
     const bool full = __ballot_sync(FULL, lane < KNN && seed >= 0) == (1u << KNN) - 1u;
     const float w = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(d)));
-    WarpList L;
+    WarpList<true> L;
     L.clear(full && w < INF ? __uint_as_float(__float_as_uint(w) + 1u) : INF);
     warp_knn(ix, px, py, pz, KNN, L, sm.ps.pool);
     // the smallest sqrtf(d2) - r; the list is in (d2, cloud index) order, so

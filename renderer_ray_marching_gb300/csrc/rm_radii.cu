@@ -402,7 +402,7 @@ k_radii_hard(IndexDev ix, HardList hard, float* __restrict__ r_sorted, int32_t* 
     const float4 q = __ldg(ix.rec + self);
     // its three nearest hold the two nearest others, and itself (unless three
     // other points coincide with it)
-    WarpList L;
+    WarpList<true> L;
     L.clear(__int_as_float(0x7f800000));
     warp_knn(ix, q.x, q.y, q.z, 3, L, pools[warp]);
     const int a = __shfl_sync(0xffffffffu, L.s, 0) == self ? 1 : 0;
@@ -570,11 +570,11 @@ k_knn(IndexDev ix, const float* __restrict__ q, int stride, int64_t m, int k,
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int64_t t = blockIdx.x * (int64_t)KNN_WARPS + warp; t < m; t += (int64_t)gridDim.x * KNN_WARPS) {
     const float* p = q + t * stride;
-    WarpList L;
+    WarpList<false> L;
     L.clear(__int_as_float(0x7f800000));
     warp_knn(ix, __ldg(p), __ldg(p + 1), __ldg(p + 2), k, L, pools[warp]);
     if (lane < k) {
-      idx_out[t * k + lane] = L.s >= 0 ? (int32_t)(unsigned)L.key : -1;
+      idx_out[t * k + lane] = L.index();
       d2_out[t * k + lane] = __uint_as_float((unsigned)(L.key >> 32));
     }
     __syncwarp();
