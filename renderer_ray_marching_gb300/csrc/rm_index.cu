@@ -610,14 +610,16 @@ __device__ __forceinline__ void split_runs(uint32_t (&k)[4], const float4* __res
 // records, colours and permutation in that order, and the groups of the
 // three (leaf 32: two) levels above the leaves that lie inside the block.
 //
-// Bound by the random 16-byte gather of the points and by the sorting
-// networks' instructions: 1.15 ms at 20M points, where the gather alone in
-// curve order, with the leaf boxes and a launch per level, took 1.48.  What
+// Bound by the random 16-byte gather of the points (2.1 GB of DRAM reads at
+// 20M points, 107 bytes a point) and by the sorting networks' instructions:
+// 0.94 ms at 20M points, where the gather alone in curve order, with the leaf
+// boxes and a launch per level, took 1.48.  Without a register cap two CTAs
+// fit on an SM and it took 1.15; three to six CTAs measured the same.  What
 // it buys at 20M points, against a Morton order: 50 instead of 74 node
 // expansions and 17.5 instead of 25.4 leaves per step of the marcher's warps
 // (24 views: 313 -> 240 ms).
 template <int LEAF>
-__global__ void __launch_bounds__(BLK_THREADS)
+__global__ void __launch_bounds__(BLK_THREADS, 3)
 k_blocks(const float4* __restrict__ pos, const float* __restrict__ radii, const uint32_t* __restrict__ order,
          int64_t n, int depth, float4* __restrict__ rec, uint32_t* __restrict__ col, int32_t* __restrict__ perm,
          float4* __restrict__ groups) {

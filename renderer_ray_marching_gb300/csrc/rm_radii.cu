@@ -309,14 +309,24 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
     while (sp > 0) {
       if (listed > REGION_LIST - 32) {
         if (++scans > REGION_SCANS<CHUNKS>) {
-          // the chunks' bounds are loose as a whole (points strewn over a
-          // dense surface of other blocks): a search for every query instead
+          // The chunks' bounds are loose as a whole (points strewn over a
+          // dense surface of other blocks): a search for every query
+          // instead.  Only coincident points stay: their bound of 0 is as
+          // tight as a search's.
+          bool stay = false;
           for (int c = 0; c < CHUNKS; ++c) {
-            hand_over(sm.d[32 * c + lane] >= 0.0f, (uint32_t)(base + 32 * c + lane), hard);
-            sm.d[32 * c + lane] = -1.0f;
+            const float d = sm.d[32 * c + lane];
+            hand_over(d > 0.0f, (uint32_t)(base + 32 * c + lane), hard);
+            if (d > 0.0f) sm.d[32 * c + lane] = -1.0f;
+            const bool some = __ballot_sync(FULL, d == 0.0f) != 0;
+            if (lane == 0) sm.chunk[c][6] = some ? 0.0f : -1.0f;
+            stay |= some;
           }
-          listed = 0;
-          break;
+          __syncwarp();
+          if (!stay) {
+            listed = 0;
+            break;
+          }
         }
         region_scan(ix, sm, base, listed);
         listed = 0;

@@ -22,6 +22,10 @@ def _cloud(kind, n):
         xyz = rng.random((n, 3)).astype(np.float32)
         xyz[rng.integers(0, n, n // 2)] = xyz[rng.integers(0, n, n // 2)]
         return xyz
+    if kind == "zeros":  # a third of the points at one place, as missing returns are stored
+        xyz = syn.make_scene(n, n_boxes=3, seed=n).xyz
+        xyz[rng.permutation(n)[: n // 3]] = 0.0
+        return xyz
     if kind == "strays":  # a dense slab and a thin layer of points above it
         xyz = rng.random((n, 3)) * [4.0, 4.0, 0.004]
         xyz[: n // 50, 2] += 0.01
@@ -30,7 +34,7 @@ def _cloud(kind, n):
     return (centres[rng.integers(0, len(centres), n)] + rng.normal(0.0, 0.01, (n, 3))).astype(np.float32)
 
 
-@pytest.mark.parametrize("kind", ["room", "grid", "twins", "strays", "clusters"])
+@pytest.mark.parametrize("kind", ["room", "grid", "twins", "zeros", "strays", "clusters"])
 @pytest.mark.parametrize("n", [1, 2, 31, 33, 127, 129, 1023, 1025, 4099, 70001])
 def test_radii_and_knn(kind, n):
     xyz = _cloud(kind, n)
