@@ -575,16 +575,19 @@ static TailList tail_list(const Ctx& c, unsigned long long* counters) {
 // 1000 at 2M points, 1400 at 20M); a ray costs the tail kernel about four
 // times its share of a full packet, so the budget is the larger the more
 // items a warp has to work off anyway, and with them the time in which a
-// slow one is hidden.  Measured optima: 200 at 0.12 items per resident warp
-// (160x120 pixels), 600 at 0.5, 900 at 2, 1000 at 5 (1067x690), 1400 at 17
-// (65 small views), 4000 to 6000 at 160 (24 views at 20M points).  Times
-// without -> with the tail kernel: 160x120 at 100k points 1.73 -> 0.65 ms,
+// slow one is hidden, and larger for a deeper tree, whose every walk opens
+// more nodes.  Measured optima: 200 at 0.12 items per resident warp (160x120
+// pixels), 600 at 0.5, 900 at 2, 1000 at 5 (1067x690), 1400 at 17 (65 small
+// views), 4000 to 6000 at 160 (24 views at 20M points); with 1010 in place of
+// 650 as the factor, one view at 20M points took 3.60 instead of 4.17 ms, but
+// 20 small views at 100k 5.51 instead of 5.28.  Times without -> with the
+// tail kernel when it was added: 160x120 at 100k points 1.73 -> 0.65 ms,
 // 320x240 at 2M 3.2 -> 1.4, 1067x690 at 2M 6.9 -> 5.6, 65 small views at 1M
 // 47.7 -> 33.9, 24 views at 20M 334 -> 316.
 constexpr int FEW = 6;
 static unsigned tail_budget(const Ctx& c, int64_t items) {
   const double per_warp = (double)items / ((double)c.sm_count * 8 * WARPS_PER_CTA);
-  return (unsigned)fmax(200.0, 650.0 * pow(per_warp, 0.38));
+  return (unsigned)fmax(200.0, (20.0 + 90.0 * c.depth) * pow(per_warp, 0.38));  // depth 7 at 100k points, 11 at 20M
 }
 
 // 524,288 rays: 6 of every tile of a 1920x1080 view, and more.  When they are
