@@ -541,7 +541,7 @@ def main():
     n_pts = int(sc.xyz.shape[0])
     radii_s = float(np.median(radii_ms)) * 1e-3
     rc = capture_figures("radii_traffic") or {}
-    radii_roof = {"bound": "hbm", "kernel": "index build + k_radii_packet",
+    radii_roof = {"bound": "hbm", "kernel": "index build + k_radii_region",
                   "achieved": round(136 * n_pts / radii_s / 1e9, 1), "peak": peak, "unit": "GB/s",
                   "frac": round(136 * n_pts / radii_s / 1e9 / peak, 4),
                   "bytes_model": "136 B/point: 16 B point read, 64 B radix sort, 32 B record gather, "
@@ -585,7 +585,7 @@ def main():
                         "l2_hit_pct": mc.get("l2_hit_pct")},
            "roofline_radii": radii_roof,
            "clocks": clk,
-           "gpu_launches": 2 * args.steps}
+           "gpu_launches": 3 * args.steps}
     if sample is not None:
         cores = os.cpu_count() or 1
         pixels, gpu_sample, panes = sample

@@ -91,7 +91,8 @@ typedef struct {
   int64_t steps;         /* total distance-function evaluations */
   int64_t hits;          /* rays that hit a sphere */
   int64_t packet_steps;  /* steps answered by a warp packet traversal */
-  int64_t solo_steps;    /* steps answered by a per-ray tree walk */
+  int64_t solo_steps;    /* steps answered for one ray alone: per-ray tree walks, and rays that
+                            left their packet for the tail kernel */
   int64_t packet_leaves; /* leaves scanned by packet traversals */
   int64_t packet_nodes;  /* tree nodes expanded by packet traversals */
   int64_t warp_steps;    /* warp-wide distance steps */
