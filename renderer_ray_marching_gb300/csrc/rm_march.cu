@@ -530,6 +530,7 @@ k_march_tail(IndexDev ix, VIEWS views, ClipBox clip, unsigned long long* __restr
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   WarpSmem& sm = smem[warp];
   const unsigned long long count = min(*tail.count, (unsigned long long)tail.cap);
+  if ((unsigned long long)blockIdx.x * WARPS_PER_CTA + warp >= count) return;  // no more warps than rays
   clear_counters(sm);
   if constexpr (std::is_same<VIEWS, PlainArgs>::value) load_view(sm.v, views);
   while (true) {
