@@ -653,26 +653,28 @@ __device__ __forceinline__ void warp_knn(const IndexDev& ix, float qx, float qy,
         at = i;
       }
     }
-    const unsigned key = (__float_as_uint(near) & ~31u) | (unsigned)lane;
+    // Only lanes whose node is needed take part, so the walk ends when no
+    // pending node is: the keys are cut to 27 bits, and which of several
+    // nodes within 32 ulps of each other comes first does not matter, but one
+    // beyond w must not hide one within it.
+    const unsigned key = near <= fminf(w, FLT_BIG) ? (__float_as_uint(near) & ~31u) | (unsigned)lane : ~0u;
     const unsigned k0 = __reduce_min_sync(FULL, key);
+    if (k0 == ~0u) break;
     const unsigned k1 = __reduce_min_sync(FULL, key == k0 ? ~0u : key);
-    const float d0 = __shfl_sync(FULL, near, k0 & 31u), d1 = __shfl_sync(FULL, near, k1 & 31u);
     const int a0 = __shfl_sync(FULL, at, k0 & 31u), a1 = __shfl_sync(FULL, at, k1 & 31u);
     // one node at a time until there is a bound (so that no more than 15
-    // entries per two levels gather before); the keys are cut to 27 bits, so
-    // the second may be the nearer by less than that
-    const bool on0 = d0 <= fminf(w, FLT_BIG), on1 = k1 != ~0u && d1 <= fminf(w, FLT_BIG) && (w < INF || !on0);
-    if (!on0 && !on1) break;
-    const int hi = on0 && on1 ? max(a0, a1) : on0 ? a0 : a1, lo = on0 && on1 ? min(a0, a1) : -1;
-    take = lo >= 0 ? 2 : 1;
+    // entries per two levels gather before)
+    const bool both = k1 != ~0u && w < INF;
+    const int hi = both ? max(a0, a1) : a0, lo = both ? min(a0, a1) : -1;
+    take = both ? 2 : 1;
     G0 = pool.code[hi];
-    G1 = lo >= 0 ? pool.code[lo] : 0;
+    G1 = both ? pool.code[lo] : 0;
     __syncwarp();
     // the last entries fill the gaps, the higher gap first
     if (lane == 0) {
       pool.code[hi] = pool.code[n - 1];
       pool.dist[hi] = pool.dist[n - 1];
-      if (lo >= 0) {
+      if (both) {
         pool.code[lo] = pool.code[n - 2];
         pool.dist[lo] = pool.dist[n - 2];
       }
