@@ -27,8 +27,9 @@
 // is taken out of the formula instead: q is as small as the ray's distance
 // from the centre, so disc = a r^2 - |q|^2 is good to 1e-10 of r^2, where
 // b^2 - a (...) in FP64 carries an error of 1e-15 b^2, 1e-9 of a
-// millimetre's square at 3 m.  Coordinates or radii outside the range where
-// floats hold such products keep FP64.
+// millimetre's square at 3 m.  Coordinates, radii or incoming gradients
+// outside the range where floats hold such products keep FP64 (a product of
+// an infinity is one; its low part would be NaN).
 #include "rm_internal.h"
 
 namespace rm {
@@ -110,11 +111,15 @@ __device__ __forceinline__ void entry_gradient(const Ray& r, const float4& c, fl
   const float d[3] = {r.dx, r.dy, r.dz};
   const Two oc[3] = {two_sum(c.x, -r.ox), two_sum(c.y, -r.oy), two_sum(c.z, -r.oz)};
   const float far = fmaxf(fmaxf(fabsf(oc[0].hi), fabsf(oc[1].hi)), fabsf(oc[2].hi));
-  if (far < 1048576.0f && rad < 1048576.0f && (rad >= 1e-9f || rad == 0.0f)) {
+  const float up = fabsf(ld);
+  Two aa = two_prod(d[0], d[0]);
+  aa = add(aa, two_prod(d[1], d[1]));
+  aa = add(aa, two_prod(d[2], d[2]));
+  // (a ray of a matrix with a fourth row can be far from unit length; NaN and
+  // infinities fail these tests)
+  if (far < 1048576.0f && rad < 1048576.0f && (rad >= 1e-9f || rad == 0.0f) && up < 1e25f &&
+      (up > 1e-25f || up == 0.0f) && aa.hi > 0.25f) {
     Two q[3], n[3];
-    Two aa = two_prod(d[0], d[0]);
-    aa = add(aa, two_prod(d[1], d[1]));
-    aa = add(aa, two_prod(d[2], d[2]));
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
       const int j = (i + 1) % 3, k = (i + 2) % 3;
@@ -144,13 +149,12 @@ __device__ __forceinline__ void entry_gradient(const Ray& r, const float4& c, fl
   const double oc0 = (double)c.x - (double)r.ox, oc1 = (double)c.y - (double)r.oy, oc2 = (double)c.z - (double)r.oz;
   const double a2 = d0 * d0 + d1 * d1 + d2 * d2, b = d0 * oc0 + d1 * oc1 + d2 * oc2;
   const double disc = b * b - a2 * (oc0 * oc0 + oc1 * oc1 + oc2 * oc2 - rr * rr);
-  const double s = (double)ld / a2;
-  const double is = disc > 0.0 ? 1.0 / sqrt(disc) : 0.0;
+  const double ia = 1.0 / a2, is = disc > 0.0 ? 1.0 / sqrt(disc) : 0.0;
   const bool in = disc > 0.0;
-  out[0] = (float)((in ? d0 - (b * d0 - a2 * oc0) * is : d0) * s);
-  out[1] = (float)((in ? d1 - (b * d1 - a2 * oc1) * is : d1) * s);
-  out[2] = (float)((in ? d2 - (b * d2 - a2 * oc2) * is : d2) * s);
-  out[3] = in ? (float)((double)ld * (-rr * is)) : 0.0f;
+  out[0] = (float)((double)ld * ((in ? d0 - (b * d0 - a2 * oc0) * is : d0) * ia));
+  out[1] = (float)((double)ld * ((in ? d1 - (b * d1 - a2 * oc1) * is : d1) * ia));
+  out[2] = (float)((double)ld * ((in ? d2 - (b * d2 - a2 * oc2) * is : d2) * ia));
+  out[3] = (float)((double)ld * (in ? -rr * is : 0.0));
 }
 
 __global__ void __launch_bounds__(256) k_backward(BackArgs a) {
