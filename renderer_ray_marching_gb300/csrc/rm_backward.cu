@@ -25,11 +25,12 @@
 // every value is an unevaluated sum of two floats (about 48 bits, T. J.
 // Dekker's double-length arithmetic with fma products), and the cancellation
 // is taken out of the formula instead: q is as small as the ray's distance
-// from the centre, so disc = a r^2 - |q|^2 is good to 1e-10 of r^2, where
-// b^2 - a (...) in FP64 carries an error of 1e-15 b^2, 1e-9 of a
-// millimetre's square at 3 m.  Coordinates, radii or incoming gradients
-// outside the range where floats hold such products keep FP64 (a product of
-// an infinity is one; its low part would be NaN).
+// from the centre, so disc = a r^2 - |q|^2 is off by 2^-45 |q| |c - o|, where
+// b^2 - a (...) in FP64 is off by 2^-52 b^2.  That is less for spheres
+// narrower than 2^-7 of their distance; the silhouettes of wider ones keep
+// FP64.  So do coordinates, radii or incoming gradients outside the range
+// where floats hold such products (a product of an infinity is one; its low
+// part would be NaN).
 #include "rm_internal.h"
 
 namespace rm {
@@ -128,22 +129,28 @@ __device__ __forceinline__ void entry_gradient(const Ray& r, const float4& c, fl
     Two disc = mul(aa, two_prod(rad, rad));
 #pragma unroll
     for (int i = 0; i < 3; ++i) disc = add(disc, neg(mul(q[i], q[i])));
-    const Two ia = mul(inv(aa), ld);
-    if (disc.hi > 0.0f) {
-      const Two is = inv_sqrt(disc);
+    // For a wide sphere near its silhouette FP64's disc is the better one (see
+    // above), and the root lets the error through; two floats are kept where
+    // it stays below 2^-24 of the result all the same.
+    const float across = fmaxf(fmaxf(fabsf(q[0].hi), fabsf(q[1].hi)), fabsf(q[2].hi));
+    if (across <= 0x1p-7f * far || fabsf(disc.hi) >= 0x1p-20f * across * far) {
+      const Two ia = mul(inv(aa), ld);
+      if (disc.hi > 0.0f) {
+        const Two is = inv_sqrt(disc);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        const int j = (i + 1) % 3, k = (i + 2) % 3;
-        n[i] = add(mul(q[k], d[j]), neg(mul(q[j], d[k])));
-        out[i] = rounded(mul(add(Two{d[i], 0.0f}, neg(mul(n[i], is))), ia));
+        for (int i = 0; i < 3; ++i) {
+          const int j = (i + 1) % 3, k = (i + 2) % 3;
+          n[i] = add(mul(q[k], d[j]), neg(mul(q[j], d[k])));
+          out[i] = rounded(mul(add(Two{d[i], 0.0f}, neg(mul(n[i], is))), ia));
+        }
+        out[3] = -rounded(mul(is, two_prod(rad, ld)));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) out[i] = rounded(mul(ia, d[i]));
+        out[3] = 0.0f;
       }
-      out[3] = -rounded(mul(is, two_prod(rad, ld)));
-    } else {
-#pragma unroll
-      for (int i = 0; i < 3; ++i) out[i] = rounded(mul(ia, d[i]));
-      out[3] = 0.0f;
+      return;
     }
-    return;
   }
   const double d0 = r.dx, d1 = r.dy, d2 = r.dz, rr = rad;
   const double oc0 = (double)c.x - (double)r.ox, oc1 = (double)c.y - (double)r.oy, oc2 = (double)c.z - (double)r.oz;
