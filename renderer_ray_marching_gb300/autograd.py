@@ -32,6 +32,7 @@ class RenderFunction(torch.autograd.Function):
             frame.rgbd = rgbd.data_ptr() + 16 * lo
             frame.hit = hit.data_ptr() + 4 * lo
             lo += v.pixels
+        renderer.wait_for_torch()  # earlier users of these blocks are done
         renderer.render_batch_into(views, frames, device=True)
         renderer.synchronize()
         rgb = rgbd[:, :3].contiguous()
@@ -57,7 +58,6 @@ class RenderFunction(torch.autograd.Function):
         gc = torch.zeros((n, 3), dtype=torch.float32, device=dev)
         gx = torch.zeros((n, 3), dtype=torch.float32, device=dev)
         gr = torch.zeros(n, dtype=torch.float32, device=dev)
-        torch.cuda.current_stream(dev).synchronize()
         ctx.renderer.backward(ctx.views, g_rgb, g_depth, hit, gc, gx, gr)
         ctx.renderer.synchronize()
         return None, None, gc, gx, gr

@@ -7,6 +7,13 @@ and ``PointcloudRayMarcher`` (``src/ray_marching.h:11-44``:
 construction from vertices/colours/radii/tree, render_to_texture).
 Arrays may be numpy arrays (host memory; the library copies) or CUDA torch
 tensors (device memory; the library works in place on its stream).
+
+The context's stream is not torch's.  A call that takes CUDA tensors, or
+allocates some for its outputs, first waits for torch's current stream: a
+tensor may still be being written there, and the caching allocator hands out
+a freed block while the work that used it is still queued.  The two calls
+that write into the caller's buffers and return without waiting
+(``render_into``, ``render_batch_into``) leave that order to the caller.
 """
 from __future__ import annotations
 
@@ -90,6 +97,8 @@ class Renderer:
         if st != _abi.RM_OK:
             raise _abi.RmError(st, "rm_ctx_create failed (is a CUDA device present?)")
         self._h = h
+        self._stream = stream
+        self._torch_stream = None  # torch's current stream as last seen
         self.device = device
         self.n = 0
 
@@ -117,6 +126,19 @@ class Renderer:
     def synchronize(self):
         self._check(self._lib.rm_synchronize(self._h))
 
+    def wait_for_torch(self):
+        """Return when the work queued on torch's current stream is done
+        (at once when the context runs on that stream itself).  Asking costs
+        2 to 3 us, waiting for an idle stream 5."""
+        raw = torch._C._cuda_getCurrentRawStream(self.device)
+        if self._stream and raw == self._stream:
+            return
+        s = self._torch_stream
+        if s is None or s.cuda_stream != raw:
+            s = self._torch_stream = torch.cuda.current_stream(self.device)
+        if not s.query():
+            s.synchronize()
+
     # -- cloud, index, radii -------------------------------------------
     def set_cloud(self, xyz, rgb=None):
         """Upload points (N x 3 or N x stride float32) and uint8 colours."""
@@ -126,6 +148,7 @@ class Renderer:
             c = None
             if rgb is not None:
                 c = rgb.to(device=x.device, dtype=torch.uint8).contiguous()
+            self.wait_for_torch()
             self._check(self._lib.rm_cloud_set(self._h, x.data_ptr(), stride,
                                                c.data_ptr() if c is not None else None, n,
                                                _abi.RM_DEVICE))
@@ -147,6 +170,7 @@ class Renderer:
         if device:
             r = torch.empty(self.n, dtype=torch.float32, device="cuda:%d" % self.device)
             nn = torch.empty(self.n, dtype=torch.int32, device=r.device)
+            self.wait_for_torch()
             self._check(self._lib.rm_radii_compute(self._h, max_radius, r.data_ptr(), nn.data_ptr(),
                                                    _abi.RM_DEVICE))
             self.synchronize()
@@ -160,6 +184,8 @@ class Renderer:
     def set_radii(self, radii, max_radius: float = 0.1):
         loc, ptr, keep = _loc_ptr(radii, np.float32)
         n = keep.shape[0] if keep is not None else 0
+        if loc == _abi.RM_DEVICE:
+            self.wait_for_torch()
         self._check(self._lib.rm_radii_set(self._h, ptr, n, max_radius, loc))
         del keep
 
@@ -170,6 +196,7 @@ class Renderer:
         if loc == _abi.RM_DEVICE:
             idx = torch.empty((m, k), dtype=torch.int32, device=keep.device)
             d2 = torch.empty((m, k), dtype=torch.float32, device=keep.device)
+            self.wait_for_torch()
             self._check(self._lib.rm_knn(self._h, ptr, stride, m, k, idx.data_ptr(), d2.data_ptr(), loc))
             self.synchronize()
             return idx, d2
@@ -210,6 +237,8 @@ class Renderer:
         """Plain form: one view, one launch.  Images have row 0 at the bottom."""
         fr, bufs = self._alloc_frame(view, outputs, device)
         v = view.to_c()
+        if device:
+            self.wait_for_torch()
         self._check(self._lib.rm_render(self._h, ctypes.byref(v), ctypes.byref(fr),
                                         _abi.RM_DEVICE if device else _abi.RM_HOST))
         if device:
@@ -235,6 +264,8 @@ class Renderer:
             fr, b = self._alloc_frame(v, outputs, device)
             frames[i] = fr
             bufs.append(b)
+        if device:
+            self.wait_for_torch()
         self.render_batch_into(views, frames, device)
         if device:
             self.synchronize()
@@ -290,6 +321,8 @@ class Renderer:
             assert isinstance(a, np.ndarray) and a.dtype == dt and a.flags.c_contiguous
             return a.ctypes.data
 
+        if dev:
+            self.wait_for_torch()
         self._check(self._lib.rm_backward(self._h, arr, len(views), p(dl_drgb, np.float32),
                                           p(dl_ddepth, np.float32), p(hit, np.int32),
                                           p(g_rgb, np.float32), p(g_xyz, np.float32),
