@@ -79,8 +79,9 @@ void throw_kernel_errors(unsigned long long count) {
     throw KernelError("kernel reported " + std::to_string(count) + " incomplete nearest-neighbour searches");
 }
 
-// Error slots: the radii/kNN kernels count failed searches at err_counter,
-// the marchers at counters[3] (stack bound or node budget exceeded).
+// Error slots: the per-lane radii kernel counts failed searches at
+// err_counter, the marchers at counters[3] (stack bound or node budget
+// exceeded); a render clears both.  The other searches cannot fail.
 void check_kernel_errors(Ctx& c) {
   unsigned long long e[2] = {0, 0};
   CK(cudaMemcpyAsync(&e[0], err_counter(c), sizeof(e[0]), cudaMemcpyDeviceToHost, c.stream));
@@ -295,14 +296,12 @@ rm_status rm_knn(rm_ctx* ctx, const float* queries, int32_t stride, int64_t m, i
       CK(cudaMemcpyAsync(dd, hd.data(), outb * 4, cudaMemcpyHostToDevice, c.stream));
       CK(cudaStreamSynchronize(c.stream));
     } else {
-      CK(cudaMemsetAsync(err_counter(c), 0, 8, c.stream));
       launch_knn(c, dq, stride, m, k, di, dd);
       CK(cudaGetLastError());
     }
     if (loc == RM_HOST) {
       CK(cudaMemcpyAsync(idx_out, di, outb * 4, cudaMemcpyDeviceToHost, c.stream));
       CK(cudaMemcpyAsync(d2_out, dd, outb * 4, cudaMemcpyDeviceToHost, c.stream));
-      if (c.n > 0) check_kernel_errors(c);
       CK(cudaStreamSynchronize(c.stream));
     }
     return RM_OK;
@@ -338,7 +337,7 @@ rm_status rm_radii_compute(rm_ctx* ctx, float max_radius, float* radii_out, int3
     CK(cudaMemcpyAsync(sc, c.scalars.p, sizeof(sc), cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));
     set_max_radius(c, (unsigned)sc[4]);
-    throw_kernel_errors(sc[8] + sc[16 + 3]);
+    throw_kernel_errors(sc[8]);
     if (loc == RM_HOST) {
       if (radii_out) CK(cudaMemcpyAsync(radii_out, dr, n * 4, cudaMemcpyDeviceToHost, c.stream));
       if (nn_out) CK(cudaMemcpyAsync(nn_out, dn, n * 4, cudaMemcpyDeviceToHost, c.stream));
