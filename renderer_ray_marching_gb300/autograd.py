@@ -20,6 +20,7 @@ class RenderFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, renderer, views, colours, xyz, radii):
         dev = colours.device
+        views = list(views)  # read again in the backward
         if len(views) == 0:
             raise RuntimeError("no views to render")
         # all views in one launch, into one buffer (a view after the other)
@@ -35,8 +36,9 @@ class RenderFunction(torch.autograd.Function):
         renderer.wait_for_torch()  # earlier users of these blocks are done
         renderer.render_batch_into(views, frames, device=True)
         renderer.synchronize()
-        rgb = rgbd[:, :3].contiguous()
-        depth = rgbd[:, 3].contiguous()
+        # copies: contiguous() of a single pixel is a view of the buffer
+        rgb = rgbd[:, :3].clone(memory_format=torch.contiguous_format)
+        depth = rgbd[:, 3].clone(memory_format=torch.contiguous_format)
         ctx.renderer = renderer
         ctx.views = views
         ctx.n = xyz.shape[0]
