@@ -271,8 +271,13 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
         }
       // A query far from the rest of its chunk (alone on its side of a gap):
       // the chunk tells little about it, and it would widen the chunk's
-      // box, so it gets a search of its own.
-      float med = active ? N.d : INF;  // the chunk's median, by a sort across the lanes
+      // box, so it gets a search of its own.  The rest is judged by the
+      // median of the queries that do not coincide with another point (to
+      // rounding): beside repeated points every other one would seem far
+      // (16M points, 60% of them repeated: 17.0 ms against 2.9).
+      const float ulp = fmaxf(fmaxf(fabsf(q.x), fabsf(q.y)), fabsf(q.z)) * 0x1p-22f;
+      const int same = __popc(__ballot_sync(FULL, active && N.d <= ulp * ulp));
+      float med = active ? N.d : INF;  // by a sort across the lanes
 #pragma unroll
       for (int size = 2; size <= 32; size *= 2)
 #pragma unroll
@@ -280,7 +285,7 @@ k_radii_region(IndexDev ix, float* __restrict__ r_sorted, int32_t* __restrict__ 
           const float o = __shfl_xor_sync(FULL, med, j);
           med = ((lane & j) == 0) == ((lane & size) == 0) ? fminf(med, o) : fmaxf(med, o);
         }
-      med = __shfl_sync(FULL, med, max(cnt - 1, 0) / 2);
+      med = __shfl_sync(FULL, med, min(same + max(cnt - same - 1, 0) / 2, 31));
       const bool lost = active && N.d < INF && N.d > REGION_LOST * med;
       hand_over(lost, (uint32_t)s, hard);
       const bool here = active && !lost;
