@@ -104,7 +104,7 @@ struct Ctx {
   DevBuf sort_counts, scan_sums;
   DevBuf bucket_i;       // cloud indices of radii on their way to cloud order
   DevBuf scalars;        // words 0-6 bounds + flag; 64-bit [4] largest radius bits, [5, 6] radii search,
-                         // [8] its errors, [16..] counters
+                         // [8] its errors, [16..31] counters; words 64-67 the curve's grid
   DevBuf staging_in, staging_out;
   DevBuf views;          // ViewDev table
   DevBuf frame_bufs;     // device outputs for host-side frames
