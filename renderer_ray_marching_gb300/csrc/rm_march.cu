@@ -593,8 +593,14 @@ static unsigned tail_budget(const Ctx& c, int64_t items) {
 
 // 524,288 rays: 6 of every tile of a 1920x1080 view, and more.  When they are
 // used up, rays stay with their items.  Reserved with the radii, since a
-// render call may be under stream capture.
-void reserve_tail(Ctx& c) { c.tail.reserve((size_t)1 << 25); }
+// render call may be under stream capture; where there is no memory for it,
+// renders go without.
+void reserve_tail(Ctx& c) {
+  try {
+    c.tail.reserve((size_t)1 << 25);
+  } catch (const OomError&) {
+  }
+}
 
 static MarchParams march_params(const Ctx& c, int64_t items) {
   MarchParams mp;
