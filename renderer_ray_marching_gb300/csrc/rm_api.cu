@@ -490,7 +490,7 @@ void enqueue_batch(Ctx& c, int n, int64_t items, const rm_launch& L) {
     cudaGraph_t g;
     CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
     CK(cudaMemcpyAsync(c.views.p, c.pinned_views, vbytes, cudaMemcpyHostToDevice, c.stream));
-    launch_prepare_views(c, c.views.ptr<ViewDev>(), n, counters(c));
+    launch_prepare_views(c, c.views.ptr<ViewDev>(), n);
     CK(cudaMemsetAsync(c.queue.p, 0, 8, c.stream));
     CK(cudaMemsetAsync(counters(c), 0, kCounters * 8, c.stream));
     CK(cudaMemsetAsync(err_counter(c), 0, 8, c.stream));
@@ -671,7 +671,7 @@ rm_status rm_backward(rm_ctx* ctx, const rm_view* views, int32_t n, const float*
     int64_t* db = (int64_t*)(si + vb);
     CK(cudaMemcpyAsync(dv, hv.data(), vb, cudaMemcpyHostToDevice, c.stream));
     CK(cudaMemcpyAsync(db, base.data(), bb, cudaMemcpyHostToDevice, c.stream));
-    launch_prepare_views(c, dv, n, counters(c));
+    launch_prepare_views(c, dv, n);
     const float* drgb = dl_drgb;
     const float* ddep = dl_ddepth;
     const int32_t* dhit = hit;

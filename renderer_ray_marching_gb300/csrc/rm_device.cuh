@@ -129,7 +129,6 @@ template <int K>
 struct KList {
   float d[K];
   int32_t s[K];   // sorted position, -1 = empty
-  float r[K];     // record .w (radius)
 };
 
 template <int K>
@@ -138,7 +137,6 @@ __device__ __forceinline__ void klist_init(KList<K>& L) {
   for (int j = 0; j < K; ++j) {
     L.d[j] = __int_as_float(0x7f800000);
     L.s[j] = -1;
-    L.r[j] = 0.0f;
   }
 }
 
@@ -151,20 +149,16 @@ __device__ __forceinline__ bool knn_before(float d, int32_t s, float dj, int32_t
 }
 
 template <int K>
-__device__ __forceinline__ void klist_insert(KList<K>& L, float d, int32_t s, float r,
-                                             const int32_t* __restrict__ perm) {
+__device__ __forceinline__ void klist_insert(KList<K>& L, float d, int32_t s, const int32_t* __restrict__ perm) {
 #pragma unroll
   for (int j = 0; j < K; ++j) {
     if (knn_before(d, s, L.d[j], L.s[j], perm)) {
       float td = L.d[j];
       int32_t ts = L.s[j];
-      float tr = L.r[j];
       L.d[j] = d;
       L.s[j] = s;
-      L.r[j] = r;
       d = td;
       s = ts;
-      r = tr;
     }
   }
 }
@@ -356,13 +350,12 @@ struct KSet {
 __device__ __forceinline__ float list_worst(const KSet& L) { return L.worst(); }
 template <int K>
 __device__ __forceinline__ float list_worst(const KList<K>& L) { return L.d[K - 1]; }
-__device__ __forceinline__ void list_consider(KSet& L, float d, int32_t s, float r, const int32_t* perm) {
-  (void)r;
+__device__ __forceinline__ void list_consider(KSet& L, float d, int32_t s, const int32_t* perm) {
   L.consider(d, s, perm);
 }
 template <int K>
-__device__ __forceinline__ void list_consider(KList<K>& L, float d, int32_t s, float r, const int32_t* perm) {
-  klist_insert<K>(L, d, s, r, perm);
+__device__ __forceinline__ void list_consider(KList<K>& L, float d, int32_t s, const int32_t* perm) {
+  klist_insert<K>(L, d, s, perm);
 }
 
 template <class List>
@@ -374,7 +367,7 @@ __device__ __forceinline__ void scan_leaf(const IndexDev& ix, int64_t leaf, floa
   for (int64_t i = start; i < end; ++i) {
     float4 c = __ldg(ix.rec + i);
     float d = d2_point(c, qx, qy, qz);
-    if (d <= list_worst(L)) list_consider(L, d, (int32_t)i, c.w, ix.perm);
+    if (d <= list_worst(L)) list_consider(L, d, (int32_t)i, ix.perm);
   }
 }
 
@@ -918,10 +911,10 @@ __device__ bool packet_knn_bf(const IndexDev& ix, bool active, float qx, float q
               }
               const int32_t s = (int32_t)start + k;
               if (fminf(fminf(d0, d1), fminf(d2, d3)) > list_worst(L)) continue;
-              if (d0 <= list_worst(L)) list_consider(L, d0, s, 0.0f, ix.perm);
-              if (d1 <= list_worst(L)) list_consider(L, d1, s + 1, 0.0f, ix.perm);
-              if (d2 <= list_worst(L)) list_consider(L, d2, s + 2, 0.0f, ix.perm);
-              if (d3 <= list_worst(L)) list_consider(L, d3, s + 3, 0.0f, ix.perm);
+              if (d0 <= list_worst(L)) list_consider(L, d0, s, ix.perm);
+              if (d1 <= list_worst(L)) list_consider(L, d1, s + 1, ix.perm);
+              if (d2 <= list_worst(L)) list_consider(L, d2, s + 2, ix.perm);
+              if (d3 <= list_worst(L)) list_consider(L, d3, s + 3, ix.perm);
             }
           }
         }

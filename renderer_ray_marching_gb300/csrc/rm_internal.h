@@ -167,7 +167,7 @@ void launch_render_batch(Ctx& c, ViewDev* views_dev, int n, int64_t total_items,
                          const rm_launch& L, unsigned long long* queue, unsigned long long* counters,
                          bool with_tail);
 void reserve_tail(Ctx& c);
-void launch_prepare_views(Ctx& c, ViewDev* views_dev, int n, unsigned long long* counters);
+void launch_prepare_views(Ctx& c, ViewDev* views_dev, int n);
 
 // rm_backward.cu
 void launch_backward(Ctx& c, const ViewDev* views_dev, int n, int64_t total_pixels,

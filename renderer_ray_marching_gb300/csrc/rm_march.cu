@@ -239,8 +239,8 @@ __device__ __forceinline__ void march_one(const IndexDev& ix, const ClipBox& cli
 // and the rays that graze an edge go on for tens of steps: with 6 or fewer
 // lanes left are 37% of the warp steps but 5% of the ray steps at 2M points.
 // Single items (rays far from everything, or spread over several surfaces)
-// took 12 ms of a view's 7, and 32 ms where the median warp of 65 small views
-// was done after 33.  So where there is a `tail` list, an item that has used
+// took 11.5 of the 11.6 ms of a 1067x690 view whose median warp was done after
+// 6.6, and 32 of the 53 ms of 65 small views.  So where there is a `tail` list, an item that has used
 // up its budget of expansions and leaves, and a late item with a few rays
 // left, hands its rays over; k_march_tail spreads them over all warps.
 template <int SEARCH>
@@ -577,14 +577,17 @@ static TailList tail_list(const Ctx& c, unsigned long long* counters) {
 // times its share of a full packet, so the budget is the larger the more
 // items a warp has to work off anyway, and with them the time in which a
 // slow one is hidden, and larger for a deeper tree, whose every walk opens
-// more nodes.  Measured optima: 200 at 0.12 items per resident warp (160x120
+// more nodes: the factor 20 + 90 * depth is 650 at 100k points and 1010 at
+// 20M.  Measured optima: 200 at 0.12 items per resident warp (160x120
 // pixels), 600 at 0.5, 900 at 2, 1000 at 5 (1067x690), 1400 at 17 (65 small
-// views), 4000 to 6000 at 160 (24 views at 20M points); with 1010 in place of
-// 650 as the factor, one view at 20M points took 3.60 instead of 4.17 ms, but
-// 20 small views at 100k 5.51 instead of 5.28.  Times without -> with the
-// tail kernel when it was added: 160x120 at 100k points 1.73 -> 0.65 ms,
-// 320x240 at 2M 3.2 -> 1.4, 1067x690 at 2M 6.9 -> 5.6, 65 small views at 1M
-// 47.7 -> 33.9, 24 views at 20M 334 -> 316.
+// views), 4000 to 6000 at 160 (24 views at 20M points); with a factor of 1010
+// instead of 650 for every tree, one view at 20M points took 3.60 instead of
+// 4.17 ms, but 20 small views at 100k 5.51 instead of 5.28.  It is the rule for
+// items of one ray per lane and 8 CTAs per SM: longer items (rays_per_lane)
+// hand over more of their rays, 14% of the steps at 4 against 2 to 3%.  Times
+// without -> with the tail kernel when it was added: 160x120 at 100k points
+// 1.73 -> 0.65 ms, 320x240 at 2M 3.2 -> 1.4, 1067x690 at 2M 6.9 -> 5.6, 65
+// small views at 1M 47.7 -> 33.9, 24 views at 20M 334 -> 316.
 constexpr int FEW = 6;
 static unsigned tail_budget(const Ctx& c, int64_t items) {
   const double per_warp = (double)items / ((double)c.sm_count * 8 * WARPS_PER_CTA);
@@ -645,8 +648,7 @@ void launch_render_plain(Ctx& c, const rm_view& v, float4* rgbd, int32_t* hit, f
   }
 }
 
-void launch_prepare_views(Ctx& c, ViewDev* views_dev, int n, unsigned long long* counters) {
-  (void)counters;
+void launch_prepare_views(Ctx& c, ViewDev* views_dev, int n) {
   k_prepare_views<<<(n + 127) / 128, 128, 0, c.stream>>>(views_dev, n);
 }
 

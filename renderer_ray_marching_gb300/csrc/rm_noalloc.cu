@@ -117,7 +117,7 @@ extern "C" rm_status rm_render_batch_noalloc(rm_ctx* ctx, const rm_view* views, 
   e = cudaMemcpyAsync(views_dev, g_host_views, (size_t)n * sizeof(ViewDev), cudaMemcpyHostToDevice, c.stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(base, 0, kHeaderBytes, c.stream);
   if (e != cudaSuccess) return fail(c, RM_ERR_CUDA, cudaGetErrorString(e));
-  launch_prepare_views(c, views_dev, n, counters);
+  launch_prepare_views(c, views_dev, n);
   launch_render_batch(c, views_dev, n, items, L, queue, counters, false);
   e = cudaGetLastError();
   unsigned long long bad = 0;

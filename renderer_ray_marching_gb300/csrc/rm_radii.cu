@@ -64,7 +64,8 @@ k_radii(IndexDev ix, float max_radius, float* __restrict__ radii_out, int32_t* _
 // Memory traffic.  Warps take their regions from a global counter in sorted
 // order, so all resident warps work inside one window of a few MB that
 // stays in L2.  Results go out in sorted order with coalesced stores;
-// k_radii_to_cloud moves them to cloud order afterwards.
+// k_to_cloud, or k_to_buckets and k_from_buckets, and k_split move them to
+// cloud order afterwards.
 constexpr int RADII_WARPS = 4;
 // Chunks per region.  Two share the descent, but make half as many, longer
 // regions: 1 against 2 chunks measured 0.12 / 0.19 ms at 500k points (search
@@ -606,7 +607,7 @@ static int blocks_for(const Ctx& c, int64_t n, int threads) {
 
 // Radii of every point: search, then cloud-order outputs, the context's
 // clamped radii, the records' radius lanes and the largest radius (on the
-// device, for read_max_radius).
+// device, for set_max_radius).
 void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
   unsigned long long* err = c.scalars.ptr<unsigned long long>() + 8;
   if (c.launch.search == 1) {
