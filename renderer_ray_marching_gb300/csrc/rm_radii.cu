@@ -571,20 +571,25 @@ __global__ void k_split(const int2* __restrict__ pairs, int64_t n, float max_rad
 }
 
 // General k-NN (k <= 32): one query per warp, the k nearest in the warp's
-// lanes (warp_knn).  The queries come in any order, so 32 of them in one
-// warp would share nothing: one query per lane, with its list in that lane's
+// lanes (warp_knn).  Where queries come in any order, 32 of them in one
+// warp share nothing: one query per lane, with its list in that lane's
 // registers, took 27.3 ms for 500k unsorted queries (k = 10, 2M points, in
-// divergent walks) where this takes 1.3, and 570 us for 1000 queries (k = 1,
+// divergent walks) where this takes 1.25, and 570 us for 1000 queries (k = 1,
 // 100k points, the latency of the longest walk) where this takes 32.
 // Issue-bound for many queries, latency-bound for few (about 8 expansions and
 // 5 batches of leaves, one after the other).
+//
+// REST: only the queries that k_knn_lanes marked are left.
 constexpr int KNN_WARPS = 4;
+constexpr int32_t KNN_LEFT = -2;
+template <bool REST>
 __global__ void __launch_bounds__(32 * KNN_WARPS)
 k_knn(IndexDev ix, const float* __restrict__ q, int stride, int64_t m, int k,
       int32_t* __restrict__ idx_out, float* __restrict__ d2_out) {
   __shared__ WarpPool pools[KNN_WARPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int64_t t = blockIdx.x * (int64_t)KNN_WARPS + warp; t < m; t += (int64_t)gridDim.x * KNN_WARPS) {
+  const int64_t step = (int64_t)gridDim.x * KNN_WARPS;
+  const auto search = [&](int64_t t) {
     const float* p = q + t * stride;
     WarpList<false> L;
     L.clear(__int_as_float(0x7f800000));
@@ -592,6 +597,89 @@ k_knn(IndexDev ix, const float* __restrict__ q, int stride, int64_t m, int k,
     if (lane < k) {
       idx_out[t * k + lane] = L.index();
       d2_out[t * k + lane] = __uint_as_float((unsigned)(L.key >> 32));
+    }
+    __syncwarp();
+  };
+  if (REST) {
+    // 32 of the warp's queries looked at together
+    for (int64_t t0 = blockIdx.x * (int64_t)KNN_WARPS + warp; t0 < m; t0 += 32 * step) {
+      const int64_t mine = t0 + lane * step;
+      unsigned left = __ballot_sync(0xffffffffu, mine < m && idx_out[mine * k] == KNN_LEFT);
+      for (; left; left &= left - 1u) search(t0 + (__ffs(left) - 1) * step);
+    }
+  } else {
+    for (int64_t t = blockIdx.x * (int64_t)KNN_WARPS + warp; t < m; t += step) search(t);
+  }
+}
+
+// k of 1 and 2 where one query per lane is the better one: 32 consecutive
+// queries that are close together walk the same nodes, and in a small tree any
+// queries do.  The warp searches for the first query's 8 nearest points; if
+// the box of the 32 is not larger than 8 times the distance of the 8th (2, 4,
+// 6 and 11 measured: the gain levels off at 8), every lane walks for its own
+// query, bounded by its distances to those points.  Other queries are left to
+// k_knn (`all`: they walk alone all the same).
+//
+// GB300, k of 1, one query per warp -> this: 3M queries in spatial order,
+// 20k points 3.18 -> 0.44 ms, 200k points 4.25 -> 0.76; a grid of 2.25M
+// queries in its own order, 20k points 3.31 -> 1.55.  1M queries in any order,
+// 100 points 0.45 -> 0.11 ms, 1000 points 0.66 -> 0.18.  (Unbounded walks of
+// lanes took 1.30, 2.78, 2.71, 0.17 and 0.50.)
+template <int K>
+__global__ void __launch_bounds__(32 * KNN_WARPS)
+k_knn_lanes(IndexDev ix, const float* __restrict__ q, int stride, int64_t m, float far2, bool all,
+            int32_t* __restrict__ idx_out, float* __restrict__ d2_out) {
+  __shared__ WarpPool pools[KNN_WARPS];
+  constexpr int NEAR = 8;
+  const unsigned FULL = 0xffffffffu;
+  const float INF = __int_as_float(0x7f800000);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int64_t t0 = (blockIdx.x * (int64_t)KNN_WARPS + warp) * 32; t0 < m; t0 += (int64_t)gridDim.x * KNN_WARPS * 32) {
+    const int64_t t = t0 + lane;
+    const bool mine = t < m;
+    const float* p = q + (mine ? t : t0) * stride;
+    const float c[3] = {__ldg(p), __ldg(p + 1), __ldg(p + 2)};
+    float diag2 = 0.0f;  // of the queries' box; not a number if one of them is not finite
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const uint32_t o = ordered_bits(c[a]);
+      const float e = __fsub_rn(from_ordered(__reduce_max_sync(FULL, o)), from_ordered(__reduce_min_sync(FULL, o)));
+      diag2 = __fmaf_rn(e, e, diag2);
+    }
+    KList<K> N;
+    klist_init<K>(N);
+    bool near = diag2 <= far2;
+    if (near) {
+      WarpList<true> L;
+      L.clear(INF);
+      warp_knn(ix, __shfl_sync(FULL, c[0], 0), __shfl_sync(FULL, c[1], 0), __shfl_sync(FULL, c[2], 0), NEAR, L,
+               pools[warp]);
+      near = diag2 <= 64.0f * L.dist(NEAR - 1);
+      // the K smallest of the lane's distances to the 8 points; placeholders
+      // one ulp above the K-th, as in KSet::restart
+      float b[2] = {INF, INF};
+#pragma unroll
+      for (int j = 0; j < NEAR; ++j) {
+        const int32_t s = __shfl_sync(FULL, L.s, j);
+        if (s < 0) continue;
+        const float d = d2_point(__ldg(ix.rec + s), c[0], c[1], c[2]);
+        b[1] = fminf(b[1], fmaxf(b[0], d));
+        b[0] = fminf(b[0], d);
+      }
+#pragma unroll
+      for (int j = 0; j < K; ++j) N.d[j] = b[K - 1] < INF ? __uint_as_float(__float_as_uint(b[K - 1]) + 1u) : INF;
+    }
+    if (near || all) {
+      if (mine) {
+        knn_search(ix, c[0], c[1], c[2], N);
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+          idx_out[t * K + j] = N.s[j] >= 0 ? __ldg(ix.perm + N.s[j]) : -1;
+          d2_out[t * K + j] = N.s[j] >= 0 ? N.d[j] : INF;
+        }
+      }
+    } else if (mine) {
+      idx_out[t * K] = KNN_LEFT;
     }
     __syncwarp();
   }
@@ -664,10 +752,31 @@ void launch_radii(Ctx& c, float max_radius, float* radii_out, int32_t* nn_out) {
 }
 
 void launch_knn(Ctx& c, const float* q, int stride, int64_t m, int k, int32_t* idx, float* d2) {
-  int64_t b = (m + KNN_WARPS - 1) / KNN_WARPS;
-  const int64_t cap = (int64_t)c.sm_count * 64;
-  if (b > cap) b = cap;
-  k_knn<<<(unsigned)b, 32 * KNN_WARPS, 0, c.stream>>>(c.index(), q, stride, m, k, idx, d2);
+  const auto grid = [&](int64_t warps) {
+    return (unsigned)std::min((warps + KNN_WARPS - 1) / KNN_WARPS, (int64_t)c.sm_count * 64);
+  };
+  // One query per lane.  Small trees: a walk's cost grows with the leaves it
+  // scans point by point, and one query per warp gets better above about
+  // 5000 points at leaf 8, 2000 at 16, 1300 at 32.  Many queries for each
+  // point: below about 4, 32 queries in spatial order span too many points,
+  // and one query per warp is as fast as unbounded walks of lanes were.
+  // Queries in any order pay 2 to 3% for the look at their boxes (1M on 20k
+  // points 1.11 -> 1.14 ms).
+  const bool small = m >= 65536 && c.n * c.cfg.leaf_size <= 40000;
+  const bool dense = m >= 262144 && m >= 4 * c.n;
+  if (k <= 2 && (small || dense)) {
+    float far2 = 0.0f;  // an eighth of the cloud's diagonal, squared lengths: no 32 queries farther apart are near
+    for (int a = 0; a < 3; ++a) far2 += (c.bounds[3 + a] - c.bounds[a]) * (c.bounds[3 + a] - c.bounds[a]);
+    const auto lanes = [&](auto kern) {
+      kern<<<grid((m + 31) / 32), 32 * KNN_WARPS, 0, c.stream>>>(c.index(), q, stride, m, far2 / 8.0f, small, idx, d2);
+    };
+    if (k == 1) lanes(k_knn_lanes<1>);
+    else lanes(k_knn_lanes<2>);
+    if (small) return;
+    k_knn<true><<<grid(m), 32 * KNN_WARPS, 0, c.stream>>>(c.index(), q, stride, m, k, idx, d2);
+    return;
+  }
+  k_knn<false><<<grid(m), 32 * KNN_WARPS, 0, c.stream>>>(c.index(), q, stride, m, k, idx, d2);
 }
 
 }  // namespace rm
