@@ -541,11 +541,15 @@ def main():
     n_pts = int(sc.xyz.shape[0])
     radii_s = float(np.median(radii_ms)) * 1e-3
     rc = capture_figures("radii_traffic") or {}
+    # bytes per point that the passes of the route move, every array of a pass once
+    spread = n_pts >= 12 << 20  # results to cloud order through buckets
+    per_pt = 31 + 22 + 76 + 47 + 24 + (76 if spread else 52) + 20
     radii_roof = {"bound": "hbm", "kernel": "index build + k_radii_region",
-                  "achieved": round(136 * n_pts / radii_s / 1e9, 1), "peak": peak, "unit": "GB/s",
-                  "frac": round(136 * n_pts / radii_s / 1e9 / peak, 4),
-                  "bytes_model": "136 B/point: 16 B point read, 64 B radix sort, 32 B record gather, "
-                                 "16 B query read, 8 B radius + neighbour write",
+                  "achieved": round(per_pt * n_pts / radii_s / 1e9, 1), "peak": peak, "unit": "GB/s",
+                  "frac": round(per_pt * n_pts / radii_s / 1e9 / peak, 4),
+                  "bytes_model": "%d B/point moved by the passes, every array once: 31 pack, 22 curve keys, 76 radix sort, "
+                                 "47 blocks and boxes, 24 search (records in, radius + neighbour out), %d to cloud order "
+                                 "and records, 20 split into the outputs" % (per_pt, 76 if spread else 52),
                   "traffic": int(rc["dram_bytes_per_query"] * n_pts) if "dram_bytes_per_query" in rc else None,
                   "dram_bytes_per_query": rc.get("dram_bytes_per_query"),
                   "query_issue_active_pct": rc.get("sm_issue_active_pct")}
