@@ -204,7 +204,41 @@ __global__ void __launch_bounds__(256) k_backward(BackArgs a) {
         if (lane + off <= last) g[k] += o;
       }
     }
-    if (h >= 0 && ((heads >> lane) & 1u)) {
+    bool write = h >= 0 && ((heads >> lane) & 1u);
+    // Interleaved runs of few points (two points pixel by pixel: 13.3 ms for 8
+    // views of 1067x690, bound by atomics on two places, now 0.88; ten points
+    // at random 5.3, now 1.4): where a point has two runs or more on average,
+    // its runs are summed as well.  Looked for in warps of 16 runs or more,
+    // and in those of 8 or more where a run in four repeats the one before the
+    // last: two thirds of an image's warps have 8 (16 views of 1M points took
+    // 4% longer with all of them looked at, and no longer like this).
+    bool mixed = __popc(heads) >= 16;
+    if (!mixed && __popc(heads) >= 8) {
+      // the hit before the previous run: handed on from run to run
+      const unsigned below = heads & ((1u << lane) - 1u);
+      const int32_t h2 = __shfl_sync(FULL, before, below ? 31 - __clz(below) : 0);
+      mixed = 4 * __popc(__ballot_sync(FULL, write && below && h == h2)) >= __popc(heads);
+    }
+    if (mixed) {
+      const unsigned runs = __ballot_sync(FULL, write);
+      const unsigned same = __match_any_sync(FULL, write ? h : -2 - lane);
+      unsigned first = __ballot_sync(FULL, write && lane == __ffs(same) - 1);
+      if (2 * __popc(first) <= __popc(runs)) {
+        write = write && ((first >> lane) & 1u);
+        for (; first; first &= first - 1u) {
+          const int src = __ffs(first) - 1;
+          const bool in = (__shfl_sync(FULL, same, src) >> lane) & 1u;
+#pragma unroll
+          for (int k = 0; k < 7; ++k) {
+            float t = in ? g[k] : 0.0f;
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(FULL, t, off);
+            if (lane == src) g[k] = t;
+          }
+        }
+      }
+    }
+    if (write) {
       atomicAdd(a.g_rgb + 3 * (int64_t)h + 0, g[0]);
       atomicAdd(a.g_rgb + 3 * (int64_t)h + 1, g[1]);
       atomicAdd(a.g_rgb + 3 * (int64_t)h + 2, g[2]);
